@@ -73,9 +73,9 @@ PR = float(np.float32(0.7))  # Pr = Sc = 0.7f (main.f:569)
 #   lapv : phi read, m_y and dm_y/dy written (+ 7 doubles/point mode tables read)
 #   assemble: vor, psi, R_om, phi, R_phi, m_y, dm_y read; rho u, rho v, rho w, vor, phi written
 #   tder : T read and written; dT/dy, lap T written
-#   post1: T, DT, rho vv, rho uv, rho vw, rho uu, rho uw, rho ww read; T, N_x, N_y, N_z written
-#   post2: u, v, w, N_x, N_y, N_z, vor, phi read; R_om, R_phi, vor, phi written
-#          (two launches, post2a and post2b, counted together as one stage)
+#   post1: T, DT read; T written (with the 00 modes' right-hand sides; small
+#          grids update T in the post2 kernel, counted here all the same)
+#   post2: u, v, w, the six products, vor, phi read; R_om, R_phi, vor, phi written
 #   psi  : drho read, psi written (+ 7 doubles/point mode tables read)
 # The passive scalar (sc) adds to zinv lap Z, dZ/dy, Z read and 4 Z
 # written; to xphys 4 Z read, 1 Z written (the twelfth output) and its
@@ -91,8 +91,8 @@ ALGO = {
     "lapv": lambda S, Z, P, w, sc, vs: S * 16 + 2 * S * w + S * 7 * 8 // 2,
     "assemble": lambda S, Z, P, w, sc, vs: 7 * S * 16 + 5 * S * w + vs * 7 * S * w,
     "tder": lambda S, Z, P, w, sc, vs: (1 + sc) * (2 * S * 16 + 2 * S * w),
-    "post1": lambda S, Z, P, w, sc, vs: 2 * S * 16 + 10 * S * w,
-    "post2": lambda S, Z, P, w, sc, vs: 6 * S * 16 + 6 * S * w,
+    "post1": lambda S, Z, P, w, sc, vs: 2 * S * 16 + S * w,
+    "post2": lambda S, Z, P, w, sc, vs: 6 * S * 16 + 9 * S * w,
     "psi": lambda S, Z, P, w, sc, vs: S * 16 + S * w + S * 7 * 8 // 2,
 }
 

@@ -226,10 +226,13 @@ int lmc_profile_read(lmc_handle *h, int nk, double *ms, int *count);
  * lmc_footprint: device bytes lmc_create would allocate for p (0 for an
  *   unsupported grid), for admission control before creating a case. */
 /* lmc_launches_per_step: kernels one RK3 step launches on this handle.
- * lmc_y_family: 1 when the handle runs the mode-parallel y kernels (one
- *   thread per (kx,kz) mode; chosen for grids with >= 16384 modes, or by
- *   LMC_YPATH=mode|warp in the environment at lmc_create), 0 for the
- *   warp-per-mode kernels. */
+ * lmc_y_family: 1 when the handle runs the kernel sequence of grids with many
+ *   (kx,kz) modes (>= 16384, or LMC_YPATH=mode in the environment at
+ *   lmc_create, whose y kernels sweep along y with one thread per mode; so do
+ *   those of pencils of at most 28 points with more than 2368 modes; and the
+ *   2014 variant, the scalar and the variable viscosity on any grid),
+ *   0 for the sequence of smaller grids (LMC_YPATH=warp forces it), whose y
+ *   kernels split every pencil over several threads. */
 int lmc_launches_per_step(lmc_handle *h);
 int lmc_y_family(lmc_handle *h);
 int lmc_use_graphs(lmc_handle *h, int on);

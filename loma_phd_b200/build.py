@@ -14,10 +14,10 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "liblomacte_b200.so")
-SOURCES = ["lmc_y_d.cu", "lmc_y_c.cu", "lmc_y_b.cu", "lmc_y_a.cu", "lmc_ytpm.cu", "lmc_fft_c.cu", "lmc_fft_b.cu",
-           "lmc_fft_a.cu", "lmc_api.cu", "lmc_dispatch.cu", "lmc_ykernels.cu", "lmc_noalloc.cu", "lmc_yop.cu", "lmc_host.cpp"]
+SOURCES = ["lmc_yc_d.cu", "lmc_yc_c.cu", "lmc_yc_b.cu", "lmc_yc_a.cu", "lmc_y00.cu", "lmc_ytpm.cu", "lmc_fft_c.cu",
+           "lmc_fft_b.cu", "lmc_fft_a.cu", "lmc_api.cu", "lmc_dispatch.cu", "lmc_ykernels.cu", "lmc_noalloc.cu", "lmc_yop.cu", "lmc_host.cpp"]
 HEADERS = ["lmc_internal.h", "lmc_kernels.cuh", "lmc_device.cuh", "lmc_fft_impl.cuh", "lmc_async.cuh",
-           "lmc_ykernels.cuh", "lmc_ylaunch.h", "lmc_ytpm.cuh", "lmc_stats.cuh"]
+           "lmc_ychunk.cuh", "lmc_ylaunch.h", "lmc_ytpm.cuh", "lmc_ysweep.cuh", "lmc_stats.cuh"]
 
 
 def nvcc() -> str:

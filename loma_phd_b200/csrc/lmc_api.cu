@@ -159,14 +159,51 @@ bool xstage_fits(const lmc::Grid &g, int scalar, int visc) {
   return need > 0 && need + 1024 <= SMEM_BLOCK_MAX;
 }
 
-// y kernels: mode-parallel (one thread per mode) once there are enough
-// modes to fill the GPU, warp-per-mode below that.  LMC_YPATH=mode|warp
-// forces one family (tests compare them).
-bool mode_parallel(int nmode) {
+// Split of the y work by the number of modes.  LMC_YPATH=mode|warp forces the
+// split of many or of few modes (tests compare them).
+bool many_modes(int nmode) {
   const char *e = std::getenv("LMC_YPATH");
   if (e && std::strcmp(e, "mode") == 0) return true;
   if (e && std::strcmp(e, "warp") == 0) return false;
   return nmode >= 16384;
+}
+
+// modes up to which the chunked y kernels take short chunks (y_geometry)
+constexpr int FEW_MODES = 8 * 2 * 148;
+
+// Blocks of the sweeps along y (lmc_ysweep.cuh), which take over from the
+// chunked kernels (not in the 2014 variant) for grids with many modes, where
+// the sweeps fill the device (an FP64 step of 12,192 modes x 193 takes 7.4 ms
+// with the chunks and 7.6 with the sweeps, one of 8,128 x 129 3.35 and
+// 4.26 ms; 32,640 x 257 with mu = T^0.7, the scalar and float2 buffers 25.7
+// and 20.6), and for short pencils, which a chunk or three hold (with the
+// scalar and mu, 3,040 to 12,192 modes: the sweeps take 0.79 to 0.86 of the
+// chunks' step at 18 rows, 0.90 to 0.93 at 24 and 0.99 to 1.09 at 33).
+int sweep_blocks(const lmc::Grid &g, int variant) {
+  const bool force = std::getenv("LMC_YPATH") != nullptr;
+  if (variant || !(many_modes(g.nmode) || (!force && g.my <= 28 && g.nmode > FEW_MODES))) return 0;
+  return (g.nmode + lmc::YS_TB - 1) / lmc::YS_TB;
+}
+// values of scratch field q of the sweeps: whole blocks of modes, fields 1
+// and 2 those of a persistent grid
+size_t sweep_scratch(int ysb, int q, const lmc::Grid &g) {
+  const int nb = (q == 1 || q == 2) && ysb > lmc::YS_PERSIST ? lmc::YS_PERSIST : ysb;
+  return (size_t)nb * lmc::YS_TB * g.my;
+}
+// Geometry of the chunked y kernels (lmc_ychunk.cuh): rows per chunk and
+// modes per block.  Short chunks where the blocks of eight modes are at most
+// two per SM, so that the length of one block's chain is what counts (2,016
+// modes x 129, FP64: 1.32 ms per step against 1.41 with nine rows; 256 x
+// 257: 0.80 against 0.88); above that nine rows, which load fewer
+// coefficients per row, and as many modes per block as 512 threads allow
+// (4,560 x 129, float2 buffers: 1.50 against 1.56 ms; 12,192 x 193, FP64:
+// 7.43 with 16 modes, 7.54 with 8, 7.87 with five rows).
+void y_geometry(lmc::Dev &d, const lmc::Grid &g) {
+  d.ysb = sweep_blocks(g, d.variant);
+  const bool few = !many_modes(g.nmode) && g.nmode <= FEW_MODES;
+  d.yC = few && (g.my + 4) / 5 * 8 <= 512 ? 5 : 9;
+  d.ync = (g.my + d.yC - 1) / d.yC;
+  d.yMB = d.yC == 5 ? 8 : d.ync * 32 <= 256 ? 32 : d.ync * 16 <= 512 ? 16 : 8;
 }
 
 // Profiling: a (start, stop) pair of events around each group of launches,
@@ -320,7 +357,6 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
     return LMC_ECUDA;
   }
   d.my = g.my; d.mgalx = g.mgalx; d.mgalz = g.mgalz; d.nkx = g.nkx; d.mz = g.mz; d.nz1 = g.nz1; d.nmode = g.nmode;
-  d.ldy = g.my | 1;
   d.zp0 = 0; d.zkn = g.nkx; d.xt0 = 0; d.xnt = 0; d.xl0 = 0; d.msum = 1;  // the whole domain
   d.ire = 1.0 / p->Re;
   d.variant = p->variant;
@@ -341,16 +377,16 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
   // y-operator tables go to the device chunk-major (see lmcd::tab)
   const int C = d.C, lpm = d.lpm, base = d.base, extra = d.extra, my = g.my;
   auto cm = [&](const std::vector<double> &T, int W) { return lmc::chunk_major(T, my, W, C, lpm, base, extra); };
-  // the 2014 variant, the passive scalar and the variable viscosity run
-  // the mode-parallel kernels
-  d.tpm = (d.variant || p->scalar || p->visc) ? 1 : mode_parallel(g.nmode);
-  const size_t pm2 = (size_t)C * 2 * 32, pm3 = (size_t)C * 3 * 32;
-  const size_t nm = d.tpm ? 0 : (size_t)g.nmode;  // chunk-major per-mode tables: warp kernels only
-  std::vector<double> PLc(nm * pm2), PUc(nm * pm3), V12c(nm * pm2);
-  // mode-fastest per-mode tables [my][band][nmode]: mode-parallel kernels only
-  const size_t nt = d.tpm ? (size_t)g.nmode * my : 0;
+  // the 2014 variant, the passive scalar and the variable viscosity take
+  // the kernel sequence of grids that sweep along y (T's update apart)
+  y_geometry(d, g);
+  d.tpm = (d.variant || p->scalar || p->visc) ? 1 : d.ysb > 0 || many_modes(g.nmode);
+  lmc::ChunkTables ct;
+  lmc::build_chunk_tables(o, d.yC, d.ync, ct);
+  // mode-fastest per-mode tables [my][band][nmode]
+  const size_t nt = (size_t)g.nmode * my;
   std::vector<double> PLt(nt * 2), PUt(nt * 3), V12t(nt * 2);
-  if (d.tpm) {
+  {
     const size_t n = (size_t)g.nmode;
 #pragma omp parallel for schedule(static)
     for (int j = 0; j < my; j++)
@@ -361,45 +397,45 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
         for (int c = 0; c < 2; c++) V12t[((size_t)j * 2 + c) * n + m] = h->pt.V12[src * 2 + c];
       }
   }
-#pragma omp parallel for schedule(static)
-  for (int m = 0; m < (int)nm; m++) {
-    std::vector<double> a(h->pt.L.begin() + (size_t)m * my * 2, h->pt.L.begin() + (size_t)(m + 1) * my * 2);
-    std::vector<double> b(h->pt.U.begin() + (size_t)m * my * 3, h->pt.U.begin() + (size_t)(m + 1) * my * 3);
-    std::vector<double> v(h->pt.V12.begin() + (size_t)m * my * 2, h->pt.V12.begin() + (size_t)(m + 1) * my * 2);
-    const std::vector<double> ca = cm(a, 2), cb = cm(b, 3), cv = cm(v, 2);
-    std::copy(ca.begin(), ca.end(), PLc.begin() + (size_t)m * pm2);
-    std::copy(cb.begin(), cb.end(), PUc.begin() + (size_t)m * pm3);
-    std::copy(cv.begin(), cv.end(), V12c.begin() + (size_t)m * pm2);
-  }
   if ((rc = dupload(h, &d.dt12, cm(o.dt12, 7))) || (rc = dupload(h, &d.dt11, cm(o.dt11, 7))) ||
-      (rc = dupload(h, &d.dt22, cm(o.dt22, 5))) || (rc = dupload(h, &d.dt21, cm(o.dt21, 5))) ||
+      (rc = dupload(h, &d.dt22, cm(o.dt22, 5))) ||
       (rc = dupload(h, &d.p1L, cm(o.p1L, 3))) || (rc = dupload(h, &d.p1U, cm(o.p1U, 4))) ||
       (rc = dupload(h, &d.p3L, cm(o.p3L, 2))) || (rc = dupload(h, &d.p3U, cm(o.p3U, 3))) ||
       (rc = dupload(h, &d.i8L, cm(o.i8L, 3))) || (rc = dupload(h, &d.i8U, cm(o.i8U, 4))) ||
       (rc = dupload(h, &d.fmap, cm(o.fmap, 1))) || (rc = dupload(h, &d.hy, o.hy)) || (rc = dupload(h, &d.trp, o.trp)) ||
-      (rc = dupload(h, &d.y, o.y)) || (rc = dupload(h, &d.ebot, cm(o.ebot, 1))) || (rc = dupload(h, &d.etop, cm(o.etop, 1))) ||
+      (rc = dupload(h, &d.y, o.y)) ||
       (rc = dupload(h, &d.k1L, o.k1L)) || (rc = dupload(h, &d.k1U, o.k1U)) || (rc = dupload(h, &d.k3L, o.k3L)) ||
       (rc = dupload(h, &d.k3U, o.k3U)) || (rc = dupload(h, &d.k8L, o.k8L)) || (rc = dupload(h, &d.k8U, o.k8U)) ||
-      (rc = dupload(h, &d.PL, PLc)) || (rc = dupload(h, &d.PU, PUc)) || (rc = dupload(h, &d.V12, V12c)) ||
       (rc = dupload(h, &d.AAinv, h->pt.AAinv)) || (rc = dupload(h, &d.k2, h->pt.k2)) || (rc = dupload(h, &d.kx, kx)) ||
       (rc = dupload(h, &d.kz, kz))) {
     lmc_destroy(h);
     return rc;
   }
-  // row form of d/dy in every family (the statistics differentiate u, v, w
-  // one thread per mode); the rest only for the mode-parallel kernels
+  // row form of d/dy (the statistics and the export differentiate one thread
+  // per mode) and of the wall derivatives, and the per-mode tables
   if ((rc = dupload(h, &d.r_dt12, o.dt12)) || (rc = dupload(h, &d.r_p1L, o.p1L)) ||
-      (rc = dupload(h, &d.r_p1U, o.p1U)) || (rc = dupload(h, &d.r_fmap, o.fmap))) {
+      (rc = dupload(h, &d.r_p1U, o.p1U)) || (rc = dupload(h, &d.r_fmap, o.fmap)) ||
+      (rc = dupload(h, &d.r_ebot, o.ebot)) || (rc = dupload(h, &d.r_etop, o.etop)) ||
+      (rc = dupload(h, &d.PLt, PLt)) || (rc = dupload(h, &d.PUt, PUt)) || (rc = dupload(h, &d.V12t, V12t))) {
     lmc_destroy(h);
     return rc;
   }
-  if (d.tpm &&
-      ((rc = dupload(h, &d.r_dt11, o.dt11)) ||
-       (rc = dupload(h, &d.r_dt22, o.dt22)) || (rc = dupload(h, &d.r_dt21, o.dt21)) ||
+  if (d.ysb &&
+      ((rc = dupload(h, &d.r_dt22, o.dt22)) || (rc = dupload(h, &d.r_dt21, o.dt21)) ||
        (rc = dupload(h, &d.r_p3L, o.p3L)) || (rc = dupload(h, &d.r_p3U, o.p3U)) ||
-       (rc = dupload(h, &d.r_ebot, o.ebot)) ||
-       (rc = dupload(h, &d.r_etop, o.etop)) || (rc = dupload(h, &d.PLt, PLt)) || (rc = dupload(h, &d.PUt, PUt)) ||
-       (rc = dupload(h, &d.V12t, V12t)))) {
+       (rc = dupload(h, &d.r_q1U, o.q1U)) || (rc = dupload(h, &d.r_q1L, o.q1L)) ||
+       (rc = dupload(h, &d.r_q3U, o.q3U)) || (rc = dupload(h, &d.r_q3L, o.q3L)))) {
+    lmc_destroy(h);
+    return rc;
+  }
+  lmc::YChunk &q = d.ct;
+  if ((rc = dupload(h, &q.fw1, ct.fw1)) || (rc = dupload(h, &q.hl1, ct.hl1)) || (rc = dupload(h, &q.bw1, ct.bw1)) ||
+      (rc = dupload(h, &q.hu1, ct.hu1)) || (rc = dupload(h, &q.fw2, ct.fw2)) || (rc = dupload(h, &q.hl2, ct.hl2)) ||
+      (rc = dupload(h, &q.bw2, ct.bw2)) || (rc = dupload(h, &q.hu2, ct.hu2)) || (rc = dupload(h, &q.fwp, ct.fwp)) ||
+      (rc = dupload(h, &q.m1L, ct.m1L)) || (rc = dupload(h, &q.q1L, ct.q1L)) || (rc = dupload(h, &q.g1L, ct.g1L)) ||
+      (rc = dupload(h, &q.m1U, ct.m1U)) || (rc = dupload(h, &q.q1U, ct.q1U)) || (rc = dupload(h, &q.g1U, ct.g1U)) ||
+      (rc = dupload(h, &q.m2L, ct.m2L)) || (rc = dupload(h, &q.q2L, ct.q2L)) || (rc = dupload(h, &q.g2L, ct.g2L)) ||
+      (rc = dupload(h, &q.m2U, ct.m2U)) || (rc = dupload(h, &q.q2U, ct.q2U)) || (rc = dupload(h, &q.g2U, ct.g2U))) {
     lmc_destroy(h);
     return rc;
   }
@@ -445,16 +481,17 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
     // partial-sum slots: one per (z tile, warp), at most mgalz tiles of
     // lmc::XW_MAX warps
     d.mpart_ld = lmc::XW_MAX * g.mgalz;
-    if ((d.visc && (rc = dalloc(h, &d.vscr, (size_t)3 * g.my))) || (rc = dalloc(h, &d.mi, (size_t)lmc::NMI * g.my)) || (rc = dalloc(h, &h->mo[0], (size_t)12 * g.my)) ||
+    if ((d.ysb && d.visc && (rc = dalloc(h, &d.vscr, (size_t)3 * g.my))) || (rc = dalloc(h, &d.mi, (size_t)lmc::NMI * g.my)) || (rc = dalloc(h, &h->mo[0], (size_t)12 * g.my)) ||
         (rc = dalloc(h, &h->mo[1], (size_t)12 * g.my)) ||
         (rc = dalloc(h, &d.mpart, (size_t)12 * g.my * d.mpart_ld))) {
       lmc_destroy(h);
       return rc;
     }
   }
-  if (d.tpm)
-    for (int q = 0; q < 5; q++)
-      if ((rc = dalloc(h, &d.ws[q], ns))) { lmc_destroy(h); return rc; }
+  if (d.ysb) {
+    for (int q = 0; q < 6; q++)
+      if ((rc = dalloc(h, &d.ws[q], sweep_scratch(d.ysb, q, g)))) { lmc_destroy(h); return rc; }
+  }
   if (d.variant &&
       ((rc = dalloc(h, &d.Told, ns)) || (rc = dalloc(h, &d.dTs, ns)) || (rc = dalloc(h, &d.RT, ns)))) {
     lmc_destroy(h);
@@ -566,6 +603,7 @@ int lmc_physical_f64(lmc_handle *h, int nplanes, const int *jplanes, double *out
   lmc::Dev e = d;
   e.prec = 0;
   e.fft64 = 0;
+  e.ysb = 0;  // Lapvdvhom with dm_y/dy written out
   const int nf = d.scalar ? 11 : 10, nq = d.scalar ? 8 : 7;
   const size_t ns = (size_t)d.nmode * d.my, nzp = (size_t)d.nkx * d.my * d.mgalz;
   const size_t nout = (size_t)nplanes * nq * d.mgalz * d.mgalx;
@@ -667,10 +705,11 @@ namespace {
 // Two independent pieces of each substep run on the second stream, beside
 // the main chain: the T derivatives and the z transforms of the inputs made
 // from T beside Lapvdvhom, the assembly of rho u_i and its z transforms
-// (neither chain reads what the other writes), and, in the mode-parallel
-// family, the psi solve beside post1 (it reads only d(rho)/dt).  The 2014
-// variant differentiates the T that its assembly saves, and takes d(rho)
-// from a transform round trip after post1, so it runs in one chain.
+// (neither chain reads what the other writes), and the 00 RHS, the updates
+// of T and Z and the psi solve beside the RK3 update of Omega_y and phi.
+// The 2014 variant differentiates the T that its assembly saves, and takes
+// d(rho) from a transform round trip after T's update, so it runs in one
+// chain.
 // The Dev of slab block r: its z transforms (kx planes, buffers Z) or its x
 // stage (lines, buffers X; the mixed form's plane sums after the last block).
 lmc::Dev block_dev(const lmc_handle *h, int r, bool xstage) {
@@ -727,8 +766,7 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
     if (cudaEventRecord(h->ev_join, s2) != cudaSuccess) return false;
     return cudaStreamWaitEvent(s, h->ev_join, 0) == cudaSuccess;
   };
-  const bool side_t = !d.variant;
-  const bool side_psi = d.tpm && !d.variant;
+  const bool side = !d.variant;
   for (int rk = 0; rk < 3; rk++) {
     if (d.prec) {  // this substep's plane sums, and the previous ones
       d.mo_cur = h->mo[h->mo_flip];
@@ -752,7 +790,7 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
       }
       if (int rc = exchange(h, true, lmc::n_in(d), s)) return rc;
     } else {
-      if (side_t) {
+      if (side) {
         if (!fork()) return LMC_ECUDA;
         run(2, s2, [&] { lmc::launch_tder(d, s2); });
         if (d.scalar) run(2, s2, [&] { lmc::launch_zder(d, s2); });
@@ -763,7 +801,7 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
       run(0, s, [&] { lmc::launch_lapv(d, s); });
       run(1, s, [&] { lmc::launch_assemble(d, rk, s); });
       if (d.visc) run(1, s, [&] { lmc::launch_sgrad(d, s); });  // the strain-rate inputs
-      if (side_t) {
+      if (side) {
         run(3, s, [&] { lmc::launch_zinv(d, s, 0, 0, 3); });
         if (d.visc) run(3, s, [&] { lmc::launch_zinv(d, s, 0, lmc::vbase(d), 6); });
         if (cudaStreamWaitEvent(s, h->ev_join, 0) != cudaSuccess) return LMC_ECUDA;
@@ -800,21 +838,24 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
       run(5, s, [&] { lmc::launch_zfwd(d, s); });
     }
     if (st_now) run(10, s, [&] { lmc::launch_stats2(d, h->st, s); });
-    if (side_psi) {  // beside post1 and post2, which neither read nor write its data
+    if (side) {  // beside the RK3 update, which neither reads nor writes what these write
       if (!fork()) return LMC_ECUDA;
-      if (d.scalar) run(5, s2, [&] { lmc::launch_zupd(d, s2); });  // Z += Delta Z
-      run(8, s2, [&] { lmc::launch_psi_main(d, rk, s2); });
-    }
-    run(6, s, [&] { lmc::launch_post1(d, rk, do_cfl, 1, s); });
-    if (d.variant) {  // d(rho) from T and Delta T (tauij2, lomacte/cross.f:877)
+      run(6, s2, [&] { lmc::launch_post1_00(d, rk, do_cfl, 1, s2); });
+      if (d.tpm) run(6, s2, [&] { lmc::launch_tupd(d, rk, s2); });   // T += Delta T
+      if (d.scalar) run(5, s2, [&] { lmc::launch_zupd(d, s2); });    // Z += Delta Z
+      run(8, s2, [&] { lmc::launch_psi(d, rk, s2); });
+      run(7, s, [&] { lmc::launch_post(d, rk, s); });
+      if (!join()) return LMC_ECUDA;
+    } else {  // the 2014 variant: d(rho) from T and Delta T (tauij2, lomacte/cross.f:877)
+      run(6, s, [&] { lmc::launch_tupd(d, rk, s); });
+      run(6, s, [&] { lmc::launch_post1_00(d, rk, do_cfl, 1, s); });
       run(3, s, [&] { lmc::launch_zinv(d, s, 1); });
       run(4, s, [&] { lmc::launch_xdrho(d, s); });
       run(5, s, [&] { lmc::launch_zfwd(d, s, 1); });
+      run(7, s, [&] { lmc::launch_post(d, rk, s); });
+      run(8, s, [&] { lmc::launch_psi(d, rk, s); });
     }
-    run(7, s, [&] { lmc::launch_post2(d, rk, s); });
-    if (side_psi && !join()) return LMC_ECUDA;
-    if (side_psi) run(8, s, [&] { lmc::launch_psi_tail(d, rk, cfl_step, s); });
-    else run(8, s, [&] { lmc::launch_psi(d, rk, cfl_step, 1, s); });
+    run(8, s, [&] { lmc::launch_psi_tail(d, rk, cfl_step, s); });
     if (d.prec) {
       d.mean_ok = 1;
       h->mo_flip = 1 - h->mo_flip;
@@ -1057,17 +1098,17 @@ size_t lmc_device_bytes(lmc_handle *h) { return h ? h->bytes : 0; }
 
 int lmc_launches_per_step(lmc_handle *h) {
   if (!h) return LMC_EINVAL;
-  // per substep: lapv, assemble, tder, zinv, xphys, zfwd, post1, post2
-  // (two kernels in the warp family), psi; the mode-parallel family adds
-  // the 00 tails of post1 and psi and runs post2 as one kernel; the mixed
-  // forms add the plane-sum reduction after xphys
-  // the 2014 variant: 14 kernels per substep (three for the d(rho) round
-  // trip, its own 00 tail) and the Deltat kernel in the first substep
+  // per substep: lapv, assemble, tder, zinv (in two launches), xphys, zfwd,
+  // the 00 RHS, the RK3 update, psi and the 00 tail; grids with many modes
+  // (and the extensions) update T in a kernel of its own; the mixed forms add
+  // the plane-sum reduction after xphys
+  // the 2014 variant: 14 kernels per substep (zinv in one launch, three for
+  // the d(rho) round trip) and the Deltat kernel in the first substep
   if (h->d.variant) return 3 * 14 + 1;
-  // the split inverse z transform adds one; the passive scalar three (its
-  // derivatives, its inverse z transforms, its update); the variable
-  // viscosity two (the strain-rate inputs and their inverse z transforms)
-  const int per = (h->d.tpm ? 11 : 10) + (h->d.prec ? 1 : 0) + 1 + (h->d.scalar ? 3 : 0) + (h->d.visc ? 2 : 0);
+  // the passive scalar adds three (its derivatives, its inverse z transforms,
+  // its update); the variable viscosity two (the strain-rate inputs and
+  // their inverse z transforms)
+  const int per = (h->d.tpm ? 12 : 11) + (h->d.prec ? 1 : 0) + (h->d.scalar ? 3 : 0) + (h->d.visc ? 2 : 0);
   return 3 * per;
 }
 
@@ -1085,10 +1126,8 @@ size_t lmc_footprint(const lmc_params *p) {
   const size_t P = (size_t)g.my * g.mgalz * g.mgalx;
   size_t b = 6 * S * 16 + P * 8;  // state, R_om, R_phi, RHS(T)
   if (p->variant) b += 3 * S * 16;  // T before the substep, Delta T, RHS(T)
-  if (p->variant || p->scalar || p->visc || mode_parallel(g.nmode))
-    b += S * 7 * 8 + (size_t)g.nmode * 5 * 8 + 5 * S * 16 + (size_t)g.my * 40 * 8;  // tables, scratch
-  else
-    b += (size_t)g.nmode * ((size_t)C * 32 * (2 + 3 + 2) + 5) * 8 + (size_t)g.my * 15 * 8;  // Poisson, d/dy rows
+  b += S * 7 * 8 + (size_t)g.nmode * 5 * 8 + (size_t)g.my * 120 * 8;  // per-mode and y tables
+  for (int q = 0; q < 6; q++) b += sweep_scratch(sweep_blocks(g, p->variant), q, g) * 16;
   if (p->scalar) {  // Z, RHS(Z), one more spectral and z-physical work buffer
     b += S * 16 + P * 8 + (p->precision == 0 ? S * 16 + Z * 16 : S * 8 + Z * 8);
     b += 2 * (size_t)g.my * 8;  // mixed sums of the 12th output
@@ -1096,7 +1135,7 @@ size_t lmc_footprint(const lmc_params *p) {
   if (p->visc) {  // spectral buffers up to 15, z-physical ones up to 14 (18 with the scalar)
     const size_t have = p->scalar ? 12 : 11, xs = 15 - have, xz = (p->scalar ? 18 : 14) - have;
     const size_t e = p->precision == 0 ? 16 : 8;
-    b += xs * S * e + xz * Z * e + 3 * (size_t)g.my * (8 + 16);  // + mixed 00 profiles and their scratch
+    b += xs * S * e + xz * Z * e + 3 * (size_t)g.my * 8;  // + mixed 00 profiles
   }
   if (p->precision == 0) b += 11 * S * 16 + 11 * Z * 16;          // FP64 work buffers
   else b += 3 * S * 16 + 11 * S * 8 + 11 * Z * 8 + 28 * (size_t)g.my * 8 + 96 * (size_t)g.my * g.mgalz * 8;

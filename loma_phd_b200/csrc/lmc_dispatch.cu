@@ -72,8 +72,7 @@ cudaError_t kernels_init(const Dev &d) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
-  const size_t need_y = (size_t)8 * d.ldy * sizeof(double2);
-  if ((size_t)limit < xphys_smem(d) + 1024 || (size_t)limit < z_smem(d) + 1024 || (size_t)limit < need_y + 1024)
+  if ((size_t)limit < xphys_smem(d) + 1024 || (size_t)limit < z_smem(d) + 1024)
     return cudaErrorInvalidValue;
   std::lock_guard<std::mutex> lock(mu);
   if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;

@@ -134,6 +134,22 @@ static void d2_row(const double *x, int j, const std::vector<int> &lo, const std
   for (int m = 0; m < nr; m++) rhs5[ro[m] + 2] = b[nl + m];
 }
 
+// A = U' L' of a band matrix with p diagonals on either side: the LU of the
+// matrix with rows and columns reversed
+static void band_ul(int n, int p, const std::vector<double> &A, std::vector<double> &U, std::vector<double> &L) {
+  const int w = 2 * p + 1;
+  std::vector<double> R((size_t)n * w), l((size_t)n * p), u((size_t)n * (p + 1));
+  for (int i = 0; i < n; i++)
+    for (int c = 0; c < w; c++) R[(size_t)i * w + c] = A[(size_t)(n - 1 - i) * w + (w - 1 - c)];
+  band_lu(n, p, p, R.data(), l.data(), u.data());
+  U.assign((size_t)n * p, 0.0);
+  L.assign((size_t)n * (p + 1), 0.0);
+  for (int i = 0; i < n; i++) {
+    for (int c = 0; c < p; c++) U[(size_t)i * p + c] = l[(size_t)(n - 1 - i) * p + c];
+    for (int c = 0; c <= p; c++) L[(size_t)i * (p + 1) + c] = u[(size_t)(n - 1 - i) * (p + 1) + c];
+  }
+}
+
 void build_yops(int my, const double *y, YOps &o) {
   if (my < 9) throw std::runtime_error("my too small");
   o.my = my;
@@ -196,6 +212,9 @@ void build_yops(int my, const double *y, YOps &o) {
   o.dt21 = lhs2;
   o.p3L.assign((size_t)my * 2, 0.0); o.p3U.assign((size_t)my * 3, 0.0);
   band_lu(my, 2, 2, lhs2.data(), o.p3L.data(), o.p3U.data());
+
+  band_ul(my, 3, lhs1, o.q1U, o.q1L);
+  band_ul(my, 2, lhs2, o.q3U, o.q3L);
 
   // fmap = 1/(dy/deta) by the first-derivative scheme (cfdiff.f:912-937).
   std::vector<double> t(my);
@@ -291,6 +310,78 @@ void build_scans(YOps &o, int lpm, int base, int extra) {
   o.k3U = scan_table(my, 2, o.p3U, true, lpm, base, extra);
   o.k8L = scan_table(my, 3, o.i8L, false, lpm, base, extra);
   o.k8U = scan_table(my, 3, o.i8U, true, lpm, base, extra);
+}
+
+// One sweep direction of a constant band solve over chunks of C rows: T
+// holds the B multipliers per row (zero past my), row r's value is
+// -sum_d T[r][d] S_d.  resp: every row's response to the state entering its
+// chunk; M, Q, G: the chunk maps, the maps from the group's start and over
+// the groups, chunks in the order of the sweep.
+static void chunk_sweep(const std::vector<double> &T, int B, int C, int nc, bool up, std::vector<double> &resp,
+                        int rw, std::vector<double> &M, std::vector<double> &Q, std::vector<double> &G) {
+  const int bb = B * B, gl = (nc + 3) / 4;
+  M.assign((size_t)nc * bb, 0.0);
+  Q.assign((size_t)nc * bb, 0.0);
+  G.assign((size_t)4 * bb, 0.0);
+  for (int i = 0; i < nc; i++) {
+    const int c = up ? nc - 1 - i : i;
+    for (int q = 0; q < B; q++) {
+      std::vector<double> S(B, 0.0);
+      S[q] = 1.0;
+      for (int t = 0; t < C; t++) {
+        const int row = c * C + (up ? C - 1 - t : t);
+        double v = 0.0;
+        for (int d = 0; d < B; d++) v -= T[(size_t)row * B + d] * S[d];
+        resp[(size_t)row * rw + q] = v;
+        for (int d = B - 1; d > 0; d--) S[d] = S[d - 1];
+        S[0] = v;
+      }
+      for (int r = 0; r < B; r++) M[(size_t)i * bb + r * B + q] = S[r];
+    }
+  }
+  for (int g = 0; g < 4; g++) {
+    std::vector<double> P(bb, 0.0);
+    for (int r = 0; r < B; r++) P[r * B + r] = 1.0;
+    for (int i = g * gl; i < (g + 1) * gl && i < nc; i++) {
+      std::copy(P.begin(), P.end(), Q.begin() + (size_t)i * bb);
+      std::vector<double> n(bb, 0.0);
+      for (int r = 0; r < B; r++)
+        for (int q = 0; q < B; q++)
+          for (int k = 0; k < B; k++) n[r * B + q] += M[(size_t)i * bb + r * B + k] * P[k * B + q];
+      P = n;
+    }
+    std::copy(P.begin(), P.end(), G.begin() + (size_t)g * bb);
+  }
+}
+
+void build_chunk_tables(const YOps &o, int C, int nc, ChunkTables &t) {
+  const int my = o.my, nr = nc * C;
+  t.fw1.assign((size_t)nr * 10, 0.0); t.hl1.assign((size_t)nr * 4, 0.0);
+  t.bw1.assign((size_t)nr * 4, 0.0); t.hu1.assign((size_t)nr * 4, 0.0);
+  t.fw2.assign((size_t)nr * 12, 0.0); t.hl2.assign((size_t)nr * 2, 0.0);
+  t.bw2.assign((size_t)nr * 4, 0.0); t.hu2.assign((size_t)nr * 2, 0.0);
+  t.fwp.assign((size_t)nr * 6, 0.0);
+  std::vector<double> L1((size_t)nr * 3, 0.0), U1((size_t)nr * 3, 0.0), L2((size_t)nr * 2, 0.0), U2((size_t)nr * 2, 0.0);
+  for (int j = 0; j < my; j++) {
+    for (int c = 0; c < 7; c++) t.fw1[(size_t)j * 10 + c] = o.dt12[(size_t)j * 7 + c];
+    for (int c = 0; c < 3; c++) t.fw1[(size_t)j * 10 + 7 + c] = L1[(size_t)j * 3 + c] = o.p1L[(size_t)j * 3 + c];
+    for (int c = 0; c < 5; c++) {
+      t.fw2[(size_t)j * 12 + c] = o.dt22[(size_t)j * 5 + c];
+      t.fw2[(size_t)j * 12 + 5 + c] = o.dt21[(size_t)j * 5 + c];
+      if (j > 0 && j < my - 1) t.fwp[(size_t)j * 6 + c] = o.dt21[(size_t)j * 5 + c];
+    }
+    for (int c = 0; c < 2; c++) t.fw2[(size_t)j * 12 + 10 + c] = L2[(size_t)j * 2 + c] = o.p3L[(size_t)j * 2 + c];
+    const double r1 = o.p1U[(size_t)j * 4], r2 = o.p3U[(size_t)j * 3];
+    t.bw1[(size_t)j * 4] = r1;
+    for (int c = 0; c < 3; c++) t.bw1[(size_t)j * 4 + 1 + c] = U1[(size_t)j * 3 + c] = r1 * o.p1U[(size_t)j * 4 + 1 + c];
+    t.bw2[(size_t)j * 4] = r2;
+    for (int c = 0; c < 2; c++) t.bw2[(size_t)j * 4 + 1 + c] = U2[(size_t)j * 2 + c] = r2 * o.p3U[(size_t)j * 3 + 1 + c];
+    t.hu1[(size_t)j * 4 + 3] = o.fmap[j];
+  }
+  chunk_sweep(L1, 3, C, nc, false, t.hl1, 4, t.m1L, t.q1L, t.g1L);
+  chunk_sweep(U1, 3, C, nc, true, t.hu1, 4, t.m1U, t.q1U, t.g1U);
+  chunk_sweep(L2, 2, C, nc, false, t.hl2, 2, t.m2L, t.q2L, t.g2L);
+  chunk_sweep(U2, 2, C, nc, true, t.hu2, 2, t.m2U, t.q2U, t.g2U);
 }
 
 // Per-mode data of the Poisson operator dt22 - k^2 dt21 with Dirichlet

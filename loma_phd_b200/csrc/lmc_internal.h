@@ -33,6 +33,10 @@ struct YOps {
   std::vector<double> dt12, dt11, dt22, dt21;     // [my][7] / [my][5]
   std::vector<double> p1L, p1U;                   // [my][3], [my][4]
   std::vector<double> p3L, p3U;                   // [my][2], [my][3]
+  // the same left sides factorised the other way round, A = U' L': U' the
+  // multipliers of rows j+1.. (unit diagonal), L' the reciprocal pivot and
+  // the sub-diagonals
+  std::vector<double> q1U, q1L, q3U, q3L;         // [my][3], [my][4], [my][2], [my][3]
   std::vector<double> i8L, i8U;                   // [my][3], [my][4]
   std::vector<double> ebot, etop;                 // dv/dy at the walls as linear functionals
   // Kogge-Stone scan tables of the chunked device solves ([5][32][B][B])
@@ -57,6 +61,13 @@ std::vector<double> chunk_major(const std::vector<double> &T, int my, int W, int
 void build_scans(YOps &ops, int lpm, int base, int extra);
 void build_poisson(const Grid &g, const YOps &ops, const double *kx,
                    const double *kz, PoissonTables &pt);
+// Tables of the chunked y solves (YChunk in lmc_kernels.cuh) for chunks of C
+// rows, nc of them.
+struct ChunkTables {
+  std::vector<double> fw1, hl1, bw1, hu1, fw2, hl2, bw2, hu2, fwp;
+  std::vector<double> m1L, q1L, g1L, m1U, q1U, g1U, m2L, q2L, g2L, m2U, q2U, g2U;
+};
+void build_chunk_tables(const YOps &ops, int C, int nc, ChunkTables &t);
 // Band helpers used by the host code (row-form LU, see build_yops).
 void band_lu(int n, int p, int q, const double *A /*[n][p+q+1]*/, double *L /*[n][p]*/,
              double *U /*[n][q+1]*/, bool singular_last = false);

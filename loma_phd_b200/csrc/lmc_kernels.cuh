@@ -6,7 +6,22 @@
 
 namespace lmc {
 
+// sweeps along y (lmc_ysweep.cuh): threads (modes) per block, and blocks of a
+// persistent grid at most
+constexpr int YS_TB = 128, YS_PERSIST = 148 * 2;
 constexpr int NWB = 18;  // work-buffer slots: 12 + 6 transform inputs at most
+
+// Tables of the chunked y solves (lmc_ychunk.cuh), rows padded with zeros to
+// whole chunks.  Row records: fw* the band product and L, hl* the response of
+// a row to the state entering its chunk in the L sweep, bw* the reciprocal
+// pivot and the super-diagonals scaled by it, hu* the response in the U
+// sweep (with fmap for d/dy), fwp the Poisson right-hand side.  Per chunk in
+// the order of the sweep: m* the chunk's map of states, q* the map from its
+// group's start, g* the map over a group of chunks.
+struct YChunk {
+  const double *fw1, *hl1, *bw1, *hu1, *fw2, *hl2, *bw2, *hu2, *fwp;
+  const double *m1L, *q1L, *g1L, *m1U, *q1U, *g1U, *m2L, *q2L, *g2L, *m2U, *q2U, *g2U;
+};
 
 // Device-side view of one case.
 //   spectral fields   complex [y][kx][kz]            (kz fastest)
@@ -21,7 +36,6 @@ struct Dev {
               // (1 inverse z, 2 x stage, 4 direct z)
   int my, mgalx, mgalz, nkx, mz, nz1, nmode;
   int lpm, base, extra, C;  // y-chunking of a pencil over the lanes of a warp
-  int ldy;                  // staging stride of a pencil (odd, >= my)
   int zb_x, kb_z;           // lines per block of the x / z transform kernels
   int smem_limit;           // opt-in shared memory per block of the device (bytes)
   int xstg;                 // 1: the x stage stages its input rows where they fit (LMC_XSTG=0: never)
@@ -34,26 +48,32 @@ struct Dev {
   double ire, peclet, cfl, hxalp, hzbet;
   double gama[3], xi[3], alpha[3], beta[3];
   // y operators: band rows and precomputed scan tables
-  const double *dt12, *dt11, *dt22, *dt21, *p1L, *p1U, *p3L, *p3U, *i8L, *i8U;
+  // in the chunk-major form of the one-warp-per-pencil solves (00 modes)
+  const double *dt12, *dt11, *dt22, *p1L, *p1U, *p3L, *p3U, *i8L, *i8U;
   const double *k1L, *k1U, *k3L, *k3U, *k8L, *k8U;
-  const double *fmap, *hy, *trp, *y, *ebot, *etop;
-  // per-mode Poisson data
-  const double *PL, *PU, *V12, *AAinv, *k2;
-  // Mode-parallel y kernels (tpm = 1, lmc_ytpm.cuh): the same operators in
-  // row form ([my][band], one row read by all threads of a warp), per-mode
-  // Poisson tables mode-fastest ([my][band][nmode]), and five FP64
-  // spectral scratch fields for the forward halves of the banded solves
-  // (the fifth is the psi solve's, which runs beside post1 and post2).
-  int tpm;
+  const double *fmap, *hy, *trp, *y;
+  // per-mode Poisson data, mode-fastest ([my][band][nmode])
+  const double *PLt, *PUt, *V12t, *AAinv, *k2;
+  // y kernels: rows per chunk, modes per block, chunks of a pencil (chosen
+  // by y_geometry in lmc_api.cu); tpm: the split of grids with many modes
+  int tpm, yC, yMB, ync;
+  YChunk ct;
+  // grids with many modes sweep along y with one thread per mode
+  // (lmc_ysweep.cuh): blocks of the persistent grid at most (0: the chunked
+  // kernels), the threads' scratch pencils [my][threads], and the tables in
+  // row form
+  int ysb;
+  double2 *ws[6], *vscr;
+  const double *r_dt22, *r_dt21, *r_p3L, *r_p3U, *r_q1U, *r_q1L, *r_q3U, *r_q3L;
   // 2014 variant (trunk/lomacte): spectral T before this substep's update,
   // its increment Delta T, and the previous substep's spectral RHS(T);
   // tsrc is the T the transforms read (scal, or Told in the variant)
   int variant;
   double2 *Told, *dTs, *RT;
   const double2 *tsrc;
-  const double *r_dt12, *r_dt11, *r_dt22, *r_dt21, *r_p1L, *r_p1U, *r_p3L, *r_p3U, *r_fmap, *r_ebot, *r_etop;
-  const double *PLt, *PUt, *V12t;
-  double2 *ws[5];
+  // row forms ([my][band]) of d/dy (statistics, export) and of the wall
+  // derivatives
+  const double *r_dt12, *r_p1L, *r_p1U, *r_fmap, *r_ebot, *r_etop;
   const double *kx, *kz;  // wavenumber per kx plane / kz index
   const double2 *twx, *twz;  // exp(-2 pi i e / N) for the x / z transform lengths
   const float2 *twxf, *twzf;  // the same in FP32 (mixed form)
@@ -80,7 +100,6 @@ struct Dev {
   // of d(rho u_i)/dx_j, see vbase); T's and Z's diffusion take T^sigma.
   int visc;
   double sigma;
-  double2 *vscr;  // [3][my] scratch of the mixed forms' exact 00 strain-rate inputs
   double *rhst;
   // device scalars: [0] Deltat, [1] dtr, [2] time, [3] rhobot, [4] rhotop
   double *scal_d;
@@ -209,10 +228,15 @@ void launch_xdrho(const Dev &d, cudaStream_t s);
 void launch_xphys(const Dev &d, int rk, int do_cfl, int do_diag, cudaStream_t s);
 void launch_zfwd(const Dev &d, cudaStream_t s, int mode = 0);
 void launch_cfl14(const Dev &d, int do_cfl, cudaStream_t s);
-void launch_post1(const Dev &d, int rk, int do_cfl, int do_diag, cudaStream_t s);
-void launch_post2(const Dev &d, int rk, cudaStream_t s);
-void launch_psi(const Dev &d, int rk, int do_cfl, int do_diag, cudaStream_t s);
-void launch_psi_main(const Dev &d, int rk, cudaStream_t s);
+// N_i, vorticity, RHS(Omega_y), RHS(phi) and their RK3 update; T += Delta T
+// apart for grids with many modes (d.tpm), inside it for the others
+void launch_post(const Dev &d, int rk, cudaStream_t s);
+void launch_tupd(const Dev &d, int rk, cudaStream_t s);
+// the 00 modes: their RHS, dm, dw, masst and the CFL Deltat after the
+// transforms; their update, rho v00, masses and the end of the step after
+// the substep's other kernels
+void launch_post1_00(const Dev &d, int rk, int do_cfl, int do_diag, cudaStream_t s);
+void launch_psi(const Dev &d, int rk, cudaStream_t s);
 void launch_psi_tail(const Dev &d, int rk, int cfl_step, cudaStream_t s);
 // reference layout [kx][kz][y] <-> device layout [y][kx][kz]
 void launch_ref2dev(const Dev &d, const double2 *in, double2 *out, cudaStream_t s);

@@ -1,0 +1,6 @@
+// y kernels for chunks of 9 rows, 32 modes per block (see lmc_ychunk.cuh).
+#include "lmc_ychunk.cuh"
+
+namespace lmc {
+template struct YC<9, 32>;
+}  // namespace lmc

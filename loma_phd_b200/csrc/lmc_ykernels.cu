@@ -1,6 +1,5 @@
-// lmc_ykernels.cu -- dispatch of the y-direction kernels to the chunk size
-// and work-buffer precision of a case, their one-time set-up, and the
-// layout transposes of the C ABI.
+// lmc_ykernels.cu -- dispatch of the y-direction kernels to the geometry of
+// a case, their one-time set-up, and the layout transposes of the C ABI.
 #include <cuda_runtime.h>
 
 #include "lmc_ylaunch.h"
@@ -41,85 +40,94 @@ __global__ void __launch_bounds__(256) k_dev2ref(int my, int nkx, int mz, const 
   }
 }
 
+// T += Delta T, Z += Delta Z (cross.f:619-627), one value per thread; the
+// mixed forms take the exact FP64 00 mode of the increment from the plane
+// sums.  V: the 2014 variant advances the spectral T with this substep's
+// RHS(T) (in the d(rho)/dt slot) and accumulates Delta T
+// (lomacte/cross.f:563-570).
+template <typename CT, bool V, bool Z>
+__global__ void __launch_bounds__(256) k_tupd(Dev d, int rk) {
+  const size_t n = (size_t)d.nmode * d.my;
+  for (size_t p = (size_t)blockIdx.x * 256 + threadIdx.x; p < n; p += (size_t)gridDim.x * 256) {
+    double2 dT = lmcd::to_d2(__ldg(wsb<CT>(d, Z ? ODZ : V ? ODRHO : ODT) + p));
+    if constexpr (sizeof(CT) == sizeof(float2))
+      if (p % d.nmode == 0) dT = make_double2(d.mo_cur[(size_t)(Z ? ODZ : ODT) * d.my + p / d.nmode] / ((double)d.mgalx * (double)d.mgalz), 0.0);
+    if constexpr (V) {
+      const double dtg = d.scal_d[0] * d.gama[rk];
+      d.RT[p] = dT;
+      dT = lmcd::cscale(dtg, dT);
+      d.dTs[p] = lmcd::cadd(d.dTs[p], dT);
+    }
+    double2 *f = Z ? d.zsc : d.scal;
+    f[p] = lmcd::cadd(f[p], dT);
+  }
+}
+
+template <bool Z>
+void tupd(const Dev &d, int rk, cudaStream_t s) {
+  const size_t n = (size_t)d.nmode * d.my;
+  const unsigned g = (unsigned)((n + 1023) / 1024);  // four values per thread
+  if (d.prec) k_tupd<float2, false, Z><<<g, 256, 0, s>>>(d, rk);
+  else if (!Z && d.variant) k_tupd<double2, true, false><<<g, 256, 0, s>>>(d, rk);
+  else k_tupd<double2, false, Z><<<g, 256, 0, s>>>(d, rk);
+}
+
 }  // namespace
 
-#define LMC_YCASE(C, CALL)                                       \
-  case C:                                                        \
-    if (d.prec) YL<C, float2>::CALL;                             \
-    else YL<C, double2>::CALL;                                   \
-    break;
-#define LMC_YDISPATCH(CALL)                                                                   \
-  switch (d.C) {                                                                              \
-    LMC_YCASE(4, CALL) LMC_YCASE(5, CALL) LMC_YCASE(7, CALL) LMC_YCASE(9, CALL)              \
-    LMC_YCASE(13, CALL) default : LMC_YCASE(17, CALL)                                         \
-  }
+void launch_tupd(const Dev &d, int rk, cudaStream_t s) { tupd<false>(d, rk, s); }
+void launch_zupd(const Dev &d, cudaStream_t s) { tupd<true>(d, 0, s); }
 
-// d.tpm selects the mode-parallel kernels (lmc_ytpm.cu) over the
-// warp-per-mode ones; the 00-mode tails always run the warp code.
+// geometry of the chunked kernels: rows per chunk and modes per block (d.yC,
+// d.yMB, chosen by y_geometry in lmc_api.cu)
+#define LMC_YC(CALL)                          \
+  do {                                        \
+    if (d.yC == 5) YC<5, 8>::CALL;            \
+    else if (d.yMB == 8) YC<9, 8>::CALL;      \
+    else if (d.yMB == 16) YC<9, 16>::CALL;    \
+    else YC<9, 32>::CALL;                     \
+  } while (0)
+
+// d.ysb: grids with many modes sweep along y instead (lmc_ysweep.cuh)
 void launch_lapv(const Dev &d, cudaStream_t s) {
-  if (d.tpm) tpm_lapv(d, s);
-  else LMC_YDISPATCH(lapv(d, s))
+  if (d.ysb) sweep_lapv(d, s);
+  else LMC_YC(lapv(d, s));
 }
 void launch_assemble(const Dev &d, int rk, cudaStream_t s) {
-  if (d.tpm) tpm_assemble(d, rk, s);
-  else LMC_YDISPATCH(assemble(d, rk, s))
+  if (d.ysb) sweep_assemble(d, rk, s);
+  else LMC_YC(assemble(d, rk, s));
 }
 void launch_tder(const Dev &d, cudaStream_t s) {
-  if (d.tpm) tpm_tder(d, s);
-  else LMC_YDISPATCH(tder(d, s))
+  if (d.ysb) sweep_tder(d, false, s);
+  else LMC_YC(tder(d, false, s));
 }
-void launch_post1(const Dev &d, int rk, int do_cfl, int do_diag, cudaStream_t s) {
-  if (d.tpm) {
-    tpm_post1(d, rk, s);
-    LMC_YDISPATCH(post1_00(d, rk, d.variant ? 0 : do_cfl, do_diag, s))
-  } else {
-    LMC_YDISPATCH(post1(d, rk, do_cfl, do_diag, s))
-  }
+void launch_zder(const Dev &d, cudaStream_t s) {
+  if (d.ysb) sweep_tder(d, true, s);
+  else LMC_YC(tder(d, true, s));
 }
-void launch_cfl14(const Dev &d, int do_cfl, cudaStream_t s) { tpm_cfl14(d, do_cfl, s); }
-void launch_post2(const Dev &d, int rk, cudaStream_t s) {
-  if (d.tpm) tpm_post2(d, rk, s);
-  else LMC_YDISPATCH(post2(d, rk, s))
+void launch_sgrad(const Dev &d, cudaStream_t s) {
+  if (d.ysb) sweep_sgrad(d, s);
+  else LMC_YC(sgrad(d, s));
 }
-// mode-parallel family, non-variant: the psi solve and its 00 tail apart,
-// so that the solve can run beside post1 on a second stream
-void launch_psi_main(const Dev &d, int rk, cudaStream_t s) { tpm_psi(d, rk, s); }
-void launch_psi_tail(const Dev &d, int rk, int cfl_step, cudaStream_t s) {
-  LMC_YDISPATCH(psi_00(d, rk, cfl_step, s))
+void launch_post(const Dev &d, int rk, cudaStream_t s) {
+  if (d.ysb) sweep_post(d, rk, s);
+  else LMC_YC(post(d, rk, !d.tpm, s));
 }
-void launch_psi(const Dev &d, int rk, int cfl_step, int do_diag, cudaStream_t s) {
-  if (d.tpm) {
-    tpm_psi(d, rk, s);
-    if (d.variant) tpm_psi00_14(d, rk, s);
-    else LMC_YDISPATCH(psi_00(d, rk, cfl_step, s))
-  } else {
-    LMC_YDISPATCH(psi(d, rk, cfl_step, do_diag, s))
-  }
-}
+void launch_psi(const Dev &d, int rk, cudaStream_t s) { LMC_YC(psi(d, rk, s)); }
 void launch_op_y(const Dev &d, int op, const double2 *in, double2 *out, double2 *out2, cudaStream_t s) {
-  if (d.tpm) {
-    tpm_op_y(d, op, in, out, out2, s);
-    return;
-  }
-  switch (d.C) {
-    case 4: YL<4, double2>::op_y(d, op, in, out, out2, s); break;
-    case 5: YL<5, double2>::op_y(d, op, in, out, out2, s); break;
-    case 7: YL<7, double2>::op_y(d, op, in, out, out2, s); break;
-    case 9: YL<9, double2>::op_y(d, op, in, out, out2, s); break;
-    case 13: YL<13, double2>::op_y(d, op, in, out, out2, s); break;
-    default: YL<17, double2>::op_y(d, op, in, out, out2, s); break;
-  }
+  LMC_YC(op_y(d, op, in, out, out2, s));
+}
+void launch_psi_tail(const Dev &d, int rk, int cfl_step, cudaStream_t s) {
+  if (d.variant) tpm_psi00_14(d, rk, s);
+  else launch_psi_00(d, rk, cfl_step, s);
 }
 
 // Opt the y kernels in to the device's largest dynamic shared memory.
 cudaError_t ykernels_init(int limit) {
-  cudaError_t e = cudaSuccess;
-#define LMC_YOPT(C)                                                          \
-  if ((e = YL<C, double2>::optin(limit)) != cudaSuccess) return e;           \
-  if ((e = YL<C, float2>::optin(limit)) != cudaSuccess) return e;
-  LMC_Y_CHUNKS(LMC_YOPT)
-#undef LMC_YOPT
-  return cudaSuccess;
+  cudaError_t e = YC<5, 8>::optin(limit);
+  if (e == cudaSuccess) e = YC<9, 8>::optin(limit);
+  if (e == cudaSuccess) e = YC<9, 16>::optin(limit);
+  if (e == cudaSuccess) e = YC<9, 32>::optin(limit);
+  return e;
 }
 
 void launch_ref2dev(const Dev &d, const double2 *in, double2 *out, cudaStream_t s) {

@@ -308,7 +308,8 @@ class Lomacte:
 
     @property
     def y_family(self) -> str:
-        """'mode' (one thread per mode) or 'warp' (one warp per mode)."""
+        """'mode' (the kernel sequence of grids with many modes) or 'warp'
+        (that of smaller grids); see lmc_y_family."""
         return "mode" if _lib().lmc_y_family(self._h) == 1 else "warp"
 
     @property
