@@ -110,21 +110,27 @@ int dupload(lmc_handle *h, const T **p, const std::vector<T> &v) {
   return LMC_OK;
 }
 
-std::vector<double2> twiddles(int n) {
-  std::vector<double2> t(n);
-  for (int k = 0; k < n; k++) {
-    const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)n;
-    t[k] = make_double2((double)cosl(a), (double)(-sinl(a)));
-  }
-  return t;
-}
-
-std::vector<float2> twiddles_f32(int n) {
-  std::vector<float2> t(n);
-  for (int k = 0; k < n; k++) {
-    const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)n;
-    t[k] = make_float2((float)cosl(a), (float)(-sinl(a)));
-  }
+// Twiddles of the passes of a transform of length n (Fft in lmc_device.cuh):
+// exp(-2 pi i m k / n) at [k M + m], k < r1, m < M = r2 r3, then
+// exp(-2 pi i m k / M) at [n + k r3 + m], k < r2, m < r3.  C: double2 or float2
+template <typename C>
+std::vector<C> fft_twiddles(int n) {
+  lmc::FftRadix f{n, n, 1, 1};
+  for (const auto &q : lmc::FFT_RADIX)
+    if (q.n == n) f = q;
+  const int M = f.r2 * f.r3;
+  std::vector<C> t;
+  auto put = [&](long long e, int len) {
+    const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)(e % len) / (long double)len;
+    C c;
+    c.x = (decltype(c.x))cosl(a);
+    c.y = (decltype(c.y))(-sinl(a));
+    t.push_back(c);
+  };
+  for (int k = 0; k < f.r1; k++)
+    for (int m = 0; m < M; m++) put((long long)k * m, n);
+  for (int k = 0; k < f.r2; k++)
+    for (int m = 0; m < f.r3; m++) put((long long)k * m, M);
   return t;
 }
 
@@ -320,10 +326,6 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
     const char *e = std::getenv("LMC_FFT64");
     d.fft64 = e ? (std::atoi(e) & 7) : 0;
   }
-  {  // LMC_XSTG=0: the x stage reads its input rows from global memory
-    const char *e = std::getenv("LMC_XSTG");
-    d.xstg = (e && std::strcmp(e, "0") == 0) ? 0 : 1;
-  }
   const lmc::Grid &g = h->g;
   int rc = LMC_OK;
   // x lengths from 24 up; z also 3 (mz = 1: a 2-D run, one kz mode)
@@ -443,7 +445,7 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
   h->pt = lmc::PoissonTables();
   {
     const double2 *tx = nullptr, *tz = nullptr;
-    if ((rc = dupload(h, &tx, twiddles(g.mgalx))) || (rc = dupload(h, &tz, twiddles(g.mgalz)))) {
+    if ((rc = dupload(h, &tx, fft_twiddles<double2>(g.mgalx))) || (rc = dupload(h, &tz, fft_twiddles<double2>(g.mgalz)))) {
       lmc_destroy(h);
       return rc;
     }
@@ -451,7 +453,7 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
     d.twz = tz;
     if (d.prec == 1) {
       const float2 *fx = nullptr, *fz = nullptr;
-      if ((rc = dupload(h, &fx, twiddles_f32(g.mgalx))) || (rc = dupload(h, &fz, twiddles_f32(g.mgalz)))) {
+      if ((rc = dupload(h, &fx, fft_twiddles<float2>(g.mgalx))) || (rc = dupload(h, &fz, fft_twiddles<float2>(g.mgalz)))) {
         lmc_destroy(h);
         return rc;
       }
@@ -478,9 +480,8 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
     }
   }
   if (d.prec) {
-    // partial-sum slots: one per (z tile, warp), at most mgalz tiles of
-    // lmc::XW_MAX warps
-    d.mpart_ld = lmc::XW_MAX * g.mgalz;
+    // partial-sum slots: one per (z tile, warp), at most mgalz tiles
+    d.mpart_ld = lmc::x_block(g.mgalx, d.prec == 1 && !(d.fft64 & 2)) / 32 * g.mgalz;
     if ((d.ysb && d.visc && (rc = dalloc(h, &d.vscr, (size_t)3 * g.my))) || (rc = dalloc(h, &d.mi, (size_t)lmc::NMI * g.my)) || (rc = dalloc(h, &h->mo[0], (size_t)12 * g.my)) ||
         (rc = dalloc(h, &h->mo[1], (size_t)12 * g.my)) ||
         (rc = dalloc(h, &d.mpart, (size_t)12 * g.my * d.mpart_ld))) {
@@ -772,8 +773,8 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
       d.mo_cur = h->mo[h->mo_flip];
       d.mo_prev = h->mo[1 - h->mo_flip];
     }
-    // the T derivatives and the inverse z transforms of the five inputs
-    // made from T (lap T, dT/dx, dT/dy, dT/dz, T) run beside Lapvdvhom, the
+    // the T derivatives and the inverse z transforms of the four inputs
+    // made from T (lap T, dT/dy, dT/dz, T) run beside Lapvdvhom, the
     // assembly of rho u_i and the z transforms of rho u_i
     if (split) {  // slab blocks: every transform after the y work, block by block
       if (!fork()) return LMC_ECUDA;
@@ -786,7 +787,7 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
       if (cudaStreamWaitEvent(s, h->ev_join, 0) != cudaSuccess) return LMC_ECUDA;
       for (int r = 0; r < h->split.n; r++) {
         const lmc::Dev e = block_dev(h, r, false);
-        run(3, s, [&] { lmc::launch_zinv(e, s, 0, 0, lmc::n_in(e)); });
+        run(3, s, [&] { lmc::launch_zinv(e, s); });
       }
       if (int rc = exchange(h, true, lmc::n_in(d), s)) return rc;
     } else {
@@ -794,8 +795,8 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
         if (!fork()) return LMC_ECUDA;
         run(2, s2, [&] { lmc::launch_tder(d, s2); });
         if (d.scalar) run(2, s2, [&] { lmc::launch_zder(d, s2); });
-        run(3, s2, [&] { lmc::launch_zinv(d, s2, 0, 3, 5); });
-        if (d.scalar) run(3, s2, [&] { lmc::launch_zinv(d, s2, 0, 8, 4); });
+        run(3, s2, [&] { lmc::launch_zinv(d, s2, 0, 3, 4); });
+        if (d.scalar) run(3, s2, [&] { lmc::launch_zinv(d, s2, 0, 7, 4); });
         if (cudaEventRecord(h->ev_join, s2) != cudaSuccess) return LMC_ECUDA;
       }
       run(0, s, [&] { lmc::launch_lapv(d, s); });
@@ -803,7 +804,7 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
       if (d.visc) run(1, s, [&] { lmc::launch_sgrad(d, s); });  // the strain-rate inputs
       if (side) {
         run(3, s, [&] { lmc::launch_zinv(d, s, 0, 0, 3); });
-        if (d.visc) run(3, s, [&] { lmc::launch_zinv(d, s, 0, lmc::vbase(d), 6); });
+        if (d.visc) run(3, s, [&] { lmc::launch_zinv(d, s, 0, lmc::vbase(d) - 1, 5); });
         if (cudaStreamWaitEvent(s, h->ev_join, 0) != cudaSuccess) return LMC_ECUDA;
       } else {
         run(2, s, [&] { lmc::launch_tder(d, s); });
@@ -1138,7 +1139,8 @@ size_t lmc_footprint(const lmc_params *p) {
     b += xs * S * e + xz * Z * e + 3 * (size_t)g.my * 8;  // + mixed 00 profiles
   }
   if (p->precision == 0) b += 11 * S * 16 + 11 * Z * 16;          // FP64 work buffers
-  else b += 3 * S * 16 + 11 * S * 8 + 11 * Z * 8 + 28 * (size_t)g.my * 8 + 96 * (size_t)g.my * g.mgalz * 8;
+  else b += 3 * S * 16 + 11 * S * 8 + 11 * Z * 8 + 28 * (size_t)g.my * 8 +
+            12 * (size_t)g.my * (lmc::x_block(g.mgalx, p->precision == 1) / 32) * g.mgalz * 8;
   b += (size_t)C * 32 * 64 * 8 + 6 * 5 * 32 * 16 * 8 + (size_t)(g.mgalx + g.mgalz) * 24;  // y tables, twiddles
   b += 64 * 16 * 64;                                              // allocation padding and scalars
   return b;

@@ -11,12 +11,8 @@
 // only the particular responses p travel between lanes; for the per-mode
 // Poisson LUs the 2x2 maps are built in registers.
 //
-// x/z transforms: four-step FFTs N = N1*N2 with both factors done by one
-// thread in registers, lines staged in shared memory with a skewed index
-// (one pad slot per N1 entries) so that both the strided and the
-// contiguous passes are free of bank conflicts.  The inverse ("nat2perm")
-// leaves the samples in a permuted order and the direct transform
-// ("perm2nat") is its transpose, so no permutation pass is needed.
+// x/z transforms: FFTs in passes of register DFTs over lines in shared memory
+// (Fft below).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -419,6 +415,30 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// Warp sums of 12 values at once: two exchanges that halve the values a lane
+// holds, then three over its last three (36 shuffles in place of 120).  The
+// lanes with (lane & 7) == 0 return the sums of values q0 .. q0+2.
+__device__ __forceinline__ int warp_sum12(const double (&a)[12], double (&v)[3]) {
+  const int lane = threadIdx.x & 31;
+  const bool h = lane & 16, g = lane & 8;
+  double b[6];
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    const double keep = h ? a[6 + i] : a[i], send = h ? a[i] : a[6 + i];
+    b[i] = keep + __shfl_xor_sync(LMC_FULL, send, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double keep = g ? b[3 + i] : b[i], send = g ? b[i] : b[3 + i];
+    v[i] = keep + __shfl_xor_sync(LMC_FULL, send, 8);
+  }
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+    for (int i = 0; i < 3; i++) v[i] += __shfl_xor_sync(LMC_FULL, v[i], off);
+  return (h ? 6 : 0) + (g ? 3 : 0);
+}
+
 #ifdef LMC_FFT_TU
 // ---------------------------------------------------------------------
 // Register DFTs of compile-time size R (natural order in and out):
@@ -426,12 +446,11 @@ __device__ __forceinline__ double warp_max(double v) {
 // Twiddles exp(-2 pi i e/R) come from a constant table (c_tw), one block
 // per size, filled by the host at initialisation.
 // ---------------------------------------------------------------------
-constexpr int TW_SIZES[] = {4, 6, 8, 9, 12, 16, 18, 24, 32, 36, 48};
+constexpr int TW_SIZES[] = {4, 6, 8, 12, 16};
 __host__ __device__ constexpr int tw_off(int R) {
-  return R == 4 ? 0 : R == 6 ? 4 : R == 8 ? 10 : R == 9 ? 18 : R == 12 ? 27 : R == 16 ? 39 : R == 18 ? 55
-       : R == 24 ? 73 : R == 32 ? 97 : R == 36 ? 129 : R == 48 ? 165 : -1;
+  return R == 4 ? 0 : R == 6 ? 4 : R == 8 ? 10 : R == 12 ? 18 : R == 16 ? 30 : -1;
 }
-constexpr int TW_TOTAL = 4 + 6 + 8 + 9 + 12 + 16 + 18 + 24 + 32 + 36 + 48;
+constexpr int TW_TOTAL = 4 + 6 + 8 + 12 + 16;
 
 static __constant__ double2 c_tw[TW_TOTAL];  // one copy per translation unit
 static __constant__ float2 c_twf[TW_TOTAL];  // the same, rounded to FP32
@@ -501,209 +520,214 @@ __device__ __forceinline__ void rdft(CT (&x)[R]) {
   }
 }
 
-// Four-step transform of nb lines of length N = N1*N2 in shared memory.
-// Line b starts at sm + b*ld; natural index n is stored at skew(n) =
-// n + n/N1.  twN[e] = exp(-2 pi i e/N).  CT is the complex type of the
-// samples and of the arithmetic (double2, or float2 in the mixed form).
-template <int N1, int N2, typename CT = double2>
-struct Four {
-  static constexpr int N = N1 * N2;
-  static constexpr int LD = N2 * (N1 + 1);  // skewed line length
-  __device__ static __forceinline__ int sk(int n) { return n + n / N1; }
-
-  // natural -> permuted: X[k2 + N2 k1] lands at skew position k1 + N1 k2
-  template <int SIGN, int U = 1>
-  __device__ static void nat2perm(CT *sm, int nb, int ld, const CT *__restrict__ twN) {
-    #pragma unroll U
-    for (int idx = threadIdx.x; idx < nb * N1; idx += blockDim.x) {
-      const int b = idx / N1, n1 = idx - b * N1;
-      CT *p = sm + (size_t)b * ld + n1;
-      CT x[N2];
+// The R = 3 Q samples of a first pass whose middle third is zero (the
+// 3/2-rule padding), x[0..Q) and x[2Q..3Q): the radix-3 stage comes first and
+// sees (a, 0, c).  Natural order in and out.
+template <int R, int SIGN, typename CT>
+__device__ __forceinline__ void dft_gap(CT (&x)[R]) {
+  constexpr int Q = R / 3;
+  using Re = typename CReal<CT>::R;
+  const Re s3 = (Re)0.86602540378443864676;
+  CT y[3][Q];
 #pragma unroll
-      for (int j = 0; j < N2; j++) x[j] = p[j * (N1 + 1)];
-      rdft<N2, SIGN>(x);
-#pragma unroll
-      for (int k = 0; k < N2; k++) {
-        CT v = x[k];
-        if (k > 0 && n1 > 0) {
-          CT w = __ldg(twN + n1 * k);
-          if (SIGN > 0) w = cconj(w);
-          v = cmul(v, w);
-        }
-        p[k * (N1 + 1)] = v;
+  for (int j = 0; j < Q; j++) {
+    const CT a = x[j], c = x[2 * Q + j];
+    const CT t = cmk<CT>(a.x - (Re)0.5 * c.x, a.y - (Re)0.5 * c.y);
+    const CT u = (SIGN > 0) ? cmk<CT>(s3 * c.y, -s3 * c.x) : cmk<CT>(-s3 * c.y, s3 * c.x);  // -SIGN i s3 c
+    y[0][j] = cadd(a, c);
+    y[1][j] = cadd(t, u);
+    y[2][j] = csub(t, u);
+    if constexpr (Q > 1)
+      if (j > 0) {
+        y[1][j] = cmul(y[1][j], ctw<R, SIGN, CT>(j));
+        y[2][j] = cmul(y[2][j], ctw<R, SIGN, CT>(2 * j));
       }
-    }
-    __syncthreads();
-    nat2perm_p2<SIGN, U>(sm, nb, ld);
+  }
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    rdft<Q, SIGN>(y[r]);
+#pragma unroll
+    for (int k = 0; k < Q; k++) x[r + 3 * k] = y[r][k];
+  }
+}
+// Its transpose: only the outputs 0..Q-1 (lo) and 2Q..3Q-1 (hi) of an R-point
+// DFT, the third that the truncation drops not formed.
+template <int R, int SIGN, typename CT>
+__device__ __forceinline__ void dft_trunc(const CT (&x)[R], CT (&lo)[R / 3], CT (&hi)[R / 3]) {
+  constexpr int Q = R / 3;
+  using Re = typename CReal<CT>::R;
+  const Re s3 = (Re)0.86602540378443864676;
+  CT y[3][Q];
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+#pragma unroll
+    for (int k = 0; k < Q; k++) y[r][k] = x[r + 3 * k];
+    rdft<Q, SIGN>(y[r]);
+  }
+#pragma unroll
+  for (int j = 0; j < Q; j++) {
+    CT a = y[0][j], b = y[1][j], c = y[2][j];
+    if constexpr (Q > 1)
+      if (j > 0) {
+        b = cmul(b, ctw<R, SIGN, CT>(j));
+        c = cmul(c, ctw<R, SIGN, CT>(2 * j));
+      }
+    const CT t = cadd(b, c), e = csub(b, c);
+    lo[j] = cadd(a, t);
+    // a + w^2 b + w^4 c with w = exp(SIGN 2 pi i / 3)
+    hi[j] = (SIGN > 0) ? cmk<CT>(a.x - (Re)0.5 * t.x + s3 * e.y, a.y - (Re)0.5 * t.y - s3 * e.x)
+                       : cmk<CT>(a.x - (Re)0.5 * t.x - s3 * e.y, a.y - (Re)0.5 * t.y + s3 * e.x);
+  }
+}
+
+// The tasks of a pass: K per line, nb lines, T threads.  With T a multiple of
+// K a thread keeps its place in the line from round to round.
+template <int K, int T, typename Fn>
+__device__ __forceinline__ void line_tasks(int nb, Fn &&fn) {
+  if constexpr (T % K == 0) {
+    const int q = threadIdx.x % K;
+    for (int b = threadIdx.x / K; b < nb; b += T / K) fn(b, q);
+  } else {
+    for (int idx = threadIdx.x; idx < nb * K; idx += T) fn(idx / K, idx % K);
+  }
+}
+
+// Transform of nb lines of length N = R1 R2 R3 in shared memory, in passes of
+// radix R1, R2, R3 (R3 = 1: two passes; R2 = 1: one), a task of a pass being
+// one register DFT.  Small radices: the two-pass form with radices up to 48
+// needs 130 to 255 registers a thread and leaves 8 to 18 warps on an SM.
+//
+// The inverse ("inv") takes natural order and leaves X[k1 + R1 k2 + R1 R2 k3]
+// at position (k1 R2 + k2) R3 + k3; the direct one ("fwd") is its transpose,
+// so the samples are never reordered.  Line b starts at sm + b*ld; position n
+// is stored at sk(n), one pad slot per run of the last pass, so that its
+// strided tasks hit different banks.  tw: exp(-2 pi i n k1 / N) at [k1 M + n],
+// M = R2 R3, then exp(-2 pi i n k2 / M) at [N + k2 R3 + n].
+// T: the threads of the block.  Every pass ends with a barrier.
+template <int R1, int R2, int R3, typename CT = double2, int T = 1>
+struct Fft {
+  static constexpr int N = R1 * R2 * R3, M = R2 * R3, Q = R1 / 3;
+  static constexpr int RUN = R3 > 1 ? R3 : R2 > 1 ? R2 : N;
+  static constexpr int LD = N + (RUN < N ? N / RUN : 0);
+  static_assert(R1 % 3 == 0, "the 3/2-rule gap must be whole sample rows of the first pass");
+  __device__ static __forceinline__ int sk(int n) { return RUN < N ? n + n / RUN : n; }
+  static constexpr int SM = M + (RUN < N ? M / RUN : 0);  // sk(k M + n) = k SM + sk(n)
+  // natural index of the sample at position n
+  __device__ static __forceinline__ int nat(int n) {
+    return n / M + R1 * ((n / R3) % R2) + R1 * R2 * (n % R3);
+  }
+  template <int SIGN>
+  __device__ static __forceinline__ CT twd(const CT *__restrict__ tw, int e) {
+    const CT w = __ldg(tw + e);
+    return SIGN > 0 ? cconj(w) : w;
   }
 
-  // the first pass of nat2perm with sample n of line b supplied by
-  // load(b, n) instead of read from shared memory (ends with a barrier)
+  // first pass of the inverse: mk(b, n1) gives the reader of task n1 of line b,
+  // rd(o, up) its sample n1 + o (o a multiple of M) in the low (n < N/3) or the
+  // high third (up; n > 2N/3: 2N/3 itself is never asked for); the rest is zero
   template <int SIGN, typename L>
-  __device__ static void nat2perm_in(CT *sm, int nb, int ld, const CT *__restrict__ twN, L &&load) {
-    for (int idx = threadIdx.x; idx < nb * N1; idx += blockDim.x) {
-      const int b = idx / N1, n1 = idx - b * N1;
-      CT *p = sm + (size_t)b * ld + n1;
-      CT x[N2];
+  __device__ static __forceinline__ void inv_p1(CT *sm, int nb, int ld, const CT *__restrict__ tw, L &&mk) {
+    line_tasks<M, T>(nb, [&](int b, int n1) {
+      const auto rd = mk(b, n1);
+      CT x[R1];
 #pragma unroll
-      for (int j = 0; j < N2; j++) x[j] = load(b, n1 + N1 * j);
-      rdft<N2, SIGN>(x);
-#pragma unroll
-      for (int k = 0; k < N2; k++) {
-        CT v = x[k];
-        if (k > 0 && n1 > 0) {
-          CT w = __ldg(twN + n1 * k);
-          if (SIGN > 0) w = cconj(w);
-          v = cmul(v, w);
-        }
-        p[k * (N1 + 1)] = v;
-      }
-    }
-    __syncthreads();
-  }
-
-  // The first pass of nat2perm for real inputs packed two per line (A + iB)
-  // under the 2/3 rule: only the N/3 lowest modes of A and B are nonzero,
-  // given as rows of nkx = N/3 complex values; the transform input is A + iB
-  // at n < nkx, its conjugate mirror at n > N - nkx and zero in the gap
-  // (the imaginary parts of mode 0 dropped, rftsingle.f:85-88).  With
-  // N2 % 3 == 0 the gap and the mirrored third are fixed ranges of the
-  // sample index j of a task (n = n1 + N1 j), so no sample is tested and
-  // the gap is never loaded.  rows(b, A, B) gives line b's two rows (false:
-  // a padding line, all zero).  Ends with a barrier.
-  template <int SIGN, typename ST, typename R>
-  __device__ static void nat2perm_in3(CT *sm, int nb, int ld, const CT *__restrict__ twN, R &&rows) {
-    static_assert(N2 % 3 == 0, "the 2/3-rule gap must be whole sample rows");
-    constexpr int J1 = N2 / 3, J2 = 2 * N2 / 3;
-    using Re = typename CReal<CT>::R;
-    auto cv = [](const ST &v) { return cmk<CT>((Re)v.x, (Re)v.y); };
-    for (int idx = threadIdx.x; idx < nb * N1; idx += blockDim.x) {
-      const int b = idx / N1, n1 = idx - b * N1;
-      CT *p = sm + (size_t)b * ld + n1;
-      const ST *A = nullptr, *B = nullptr;
-      const bool ok = rows(b, A, B);
-      CT x[N2];
-#pragma unroll
-      for (int j = 0; j < N2; j++) x[j] = cz<CT>();
-      if (ok) {
-#pragma unroll
-        for (int j = 0; j < J1; j++) {  // A + iB, n = n1 + N1 j < nkx
-          const int n = n1 + N1 * j;
-          const CT a = cv(A[n]), c = cv(B[n]);
-          x[j] = (j == 0 && n1 == 0) ? cmk<CT>(a.x, c.x) : cmk<CT>(a.x - c.y, a.y + c.x);
-        }
-#pragma unroll
-        for (int j = J2; j < N2; j++) {  // conj(A) + i conj(B) at k = N - n < nkx
-          const int k = N - n1 - N1 * j;
-          if (j > J2 || n1 > 0) {
-            const CT a = cv(A[k]), c = cv(B[k]);
-            x[j] = cmk<CT>(a.x + c.y, c.x - a.y);
-          }
-        }
-      }
-      rdft<N2, SIGN>(x);
-#pragma unroll
-      for (int k = 0; k < N2; k++) {
-        CT v = x[k];
-        if (k > 0 && n1 > 0) {
-          CT w = __ldg(twN + n1 * k);
-          if (SIGN > 0) w = cconj(w);
-          v = cmul(v, w);
-        }
-        p[k * (N1 + 1)] = v;
-      }
-    }
-    __syncthreads();
-  }
-
-  // The first pass of nat2perm for the 3/2-padded z lines read straight
-  // from their spectral rows: sample n of line b is coefficient n (n < N/3),
-  // zero (the padding N/3 .. 2N/3) or coefficient n - N/3 - 1 (the negative
-  // wavenumbers, n > 2N/3); get(b, k) returns coefficient k of line b.
-  // N2 % 3 == 0, so the three ranges are fixed ranges of the sample row j.
-  // Ends with a barrier.
-  template <int SIGN, typename G>
-  __device__ static void nat2perm_zin(CT *sm, int nb, int ld, const CT *__restrict__ twN, G &&get) {
-    static_assert(N2 % 3 == 0, "the padding gap must be whole sample rows");
-    constexpr int J1 = N2 / 3, J2 = 2 * N2 / 3, SH = N / 3 + 1;
-    for (int idx = threadIdx.x; idx < nb * N1; idx += blockDim.x) {
-      const int b = idx / N1, n1 = idx - b * N1;
-      CT *p = sm + (size_t)b * ld + n1;
-      CT x[N2];
-#pragma unroll
-      for (int j = 0; j < N2; j++) {
-        const int n = n1 + N1 * j;
-        if (j < J1) x[j] = get(b, n);
-        else if (j > J2 || (j == J2 && n1 > 0)) x[j] = get(b, n - SH);
+      for (int j = 0; j < R1; j++) {
+        if (j < Q) x[j] = rd(M * j, false);
+        else if (j > 2 * Q || (j == 2 * Q && n1 > 0)) x[j] = rd(M * j, true);
         else x[j] = cz<CT>();
       }
-      rdft<N2, SIGN>(x);
+      dft_gap<R1, SIGN>(x);
+      CT *p = sm + (size_t)b * ld + sk(n1);
+      const CT *t = tw + n1;
 #pragma unroll
-      for (int k = 0; k < N2; k++) {
-        CT v = x[k];
-        if (k > 0 && n1 > 0) {
-          CT w = __ldg(twN + n1 * k);
-          if (SIGN > 0) w = cconj(w);
-          v = cmul(v, w);
-        }
-        p[k * (N1 + 1)] = v;
-      }
-    }
+      for (int k = 0; k < R1; k++) p[k * SM] = (k > 0 && M > 1) ? cmul(x[k], twd<SIGN>(t, k * M)) : x[k];
+    });
     __syncthreads();
   }
-
-  // the second pass of nat2perm (ends with a barrier)
-  template <int SIGN, int U = 1>
-  __device__ static void nat2perm_p2(CT *sm, int nb, int ld) {
-    #pragma unroll U
-    for (int idx = threadIdx.x; idx < nb * N2; idx += blockDim.x) {
-      const int b = idx / N2, k2 = idx - b * N2;
-      CT *p = sm + (size_t)b * ld + k2 * (N1 + 1);
-      CT x[N1];
+  // second pass of the inverse (of the whole transform if R3 = 1)
+  template <int SIGN>
+  __device__ static __forceinline__ void inv_p2(CT *sm, int nb, int ld, const CT *__restrict__ tw) {
+    if constexpr (R2 > 1) {
+      line_tasks<R1 * R3, T>(nb, [&](int b, int q) {
+        const int k1 = q / R3, n2 = q - k1 * R3;
+        CT *p = sm + (size_t)b * ld + k1 * SM + n2;
+        constexpr int ST = R3 > 1 ? R3 + 1 : 1;  // sk(R3)
+        const CT *t = tw + N + n2;
+        CT x[R2];
 #pragma unroll
-      for (int j = 0; j < N1; j++) x[j] = p[j];
-      rdft<N1, SIGN>(x);
+        for (int j = 0; j < R2; j++) x[j] = p[j * ST];
+        rdft<R2, SIGN>(x);
 #pragma unroll
-      for (int j = 0; j < N1; j++) p[j] = x[j];
-    }
-    __syncthreads();
-  }
-
-  // permuted -> natural (transpose of nat2perm)
-  template <int SIGN, int U = 1>
-  __device__ static void perm2nat(CT *sm, int nb, int ld, const CT *__restrict__ twN) {
-    #pragma unroll U
-    for (int idx = threadIdx.x; idx < nb * N2; idx += blockDim.x) {
-      const int b = idx / N2, k2 = idx - b * N2;
-      CT *p = sm + (size_t)b * ld + k2 * (N1 + 1);
-      CT x[N1];
-#pragma unroll
-      for (int j = 0; j < N1; j++) x[j] = p[j];
-      rdft<N1, SIGN>(x);
-#pragma unroll
-      for (int j = 0; j < N1; j++) {
-        CT v = x[j];
-        if (j > 0 && k2 > 0) {
-          CT w = __ldg(twN + j * k2);
-          if (SIGN > 0) w = cconj(w);
-          v = cmul(v, w);
+        for (int k = 0; k < R2; k++) {
+          CT v = x[k];
+          if (k > 0 && R3 > 1) v = cmul(v, twd<SIGN>(t, k * R3));
+          p[k * ST] = v;
         }
-        p[j] = v;
-      }
+      });
+      __syncthreads();
     }
-    __syncthreads();
-    #pragma unroll U
-    for (int idx = threadIdx.x; idx < nb * N1; idx += blockDim.x) {
-      const int b = idx / N1, n1 = idx - b * N1;
-      CT *p = sm + (size_t)b * ld + n1;
-      CT x[N2];
+  }
+  // last of three passes of the inverse
+  template <int SIGN>
+  __device__ static __forceinline__ void inv_p3(CT *sm, int nb, int ld) {
+    if constexpr (R3 > 1) {
+      line_tasks<R1 * R2, T>(nb, [&](int b, int q) {
+        CT *p = sm + (size_t)b * ld + q * (R3 + 1);
+        CT x[R3];
 #pragma unroll
-      for (int j = 0; j < N2; j++) x[j] = p[j * (N1 + 1)];
-      rdft<N2, SIGN>(x);
+        for (int j = 0; j < R3; j++) x[j] = p[j];
+        rdft<R3, SIGN>(x);
 #pragma unroll
-      for (int j = 0; j < N2; j++) p[j * (N1 + 1)] = x[j];
+        for (int j = 0; j < R3; j++) p[j] = x[j];
+      });
+      __syncthreads();
     }
-    __syncthreads();
+  }
+  // the transposes
+  template <int SIGN>
+  __device__ static __forceinline__ void fwd_p3(CT *sm, int nb, int ld, const CT *__restrict__ tw) {
+    if constexpr (R3 > 1) {
+      line_tasks<R1 * R2, T>(nb, [&](int b, int q) {
+        const int k2 = q % R2;
+        CT *p = sm + (size_t)b * ld + q * (R3 + 1);
+        const CT *t = tw + N + k2 * R3;
+        CT x[R3];
+#pragma unroll
+        for (int j = 0; j < R3; j++) x[j] = p[j];
+        rdft<R3, SIGN>(x);
+#pragma unroll
+        for (int j = 0; j < R3; j++) p[j] = (j > 0) ? cmul(x[j], twd<SIGN>(t, j)) : x[j];
+      });
+      __syncthreads();
+    }
+  }
+  template <int SIGN>
+  __device__ static __forceinline__ void fwd_p2(CT *sm, int nb, int ld, const CT *__restrict__ tw) {
+    if constexpr (R2 > 1) {
+      line_tasks<R1 * R3, T>(nb, [&](int b, int q) {
+        const int k1 = q / R3, n2 = q - k1 * R3;
+        CT *p = sm + (size_t)b * ld + k1 * SM + n2;
+        constexpr int ST = R3 > 1 ? R3 + 1 : 1;
+        const CT *t = tw + k1 * M + n2;
+        CT x[R2];
+#pragma unroll
+        for (int j = 0; j < R2; j++) x[j] = p[j * ST];
+        rdft<R2, SIGN>(x);
+#pragma unroll
+        for (int j = 0; j < R2; j++) p[j * ST] = cmul(x[j], twd<SIGN>(t, j * R3));
+      });
+      __syncthreads();
+    }
+  }
+  // last pass of the direct transform for one task n1 of a line: outputs n1 +
+  // M j, lo for j < Q and hi for j >= 2 Q
+  template <int SIGN>
+  __device__ static __forceinline__ void fwd_p1(const CT *line, int n1, CT (&lo)[Q], CT (&hi)[Q]) {
+    CT x[R1];
+    line += sk(n1);
+#pragma unroll
+    for (int k = 0; k < R1; k++) x[k] = line[k * SM];
+    dft_trunc<R1, SIGN>(x, lo, hi);
   }
 };
 

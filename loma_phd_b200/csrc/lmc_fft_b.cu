@@ -1,5 +1,6 @@
-// Transform kernels for lengths 144..384 (see lmc_fft_impl.cuh).
+// Transform kernels for lengths 144..384 (see lmc_fft_impl.cuh;
+// the radices are those of FFT_RADIX).
 #define LMC_FFT_NS fft_b
 #include "lmc_fft_impl.cuh"
-#define LMC_FFT_SIZES(X) X(144, 12, 12) X(192, 12, 16) X(288, 16, 18) X(384, 16, 24)
+#define LMC_FFT_SIZES(X) X(144, 12, 12, 1) X(192, 12, 16, 1) X(288, 6, 6, 8) X(384, 6, 8, 8)
 LMC_FFT_TU_BODY(b)

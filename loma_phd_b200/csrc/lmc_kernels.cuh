@@ -9,6 +9,14 @@ namespace lmc {
 // sweeps along y (lmc_ysweep.cuh): threads (modes) per block, and blocks of a
 // persistent grid at most
 constexpr int YS_TB = 128, YS_PERSIST = 148 * 2;
+// Radices of the transform lengths (Fft in lmc_device.cuh): the first is a
+// multiple of 3, so that the 3/2-rule gap is whole sample rows.
+struct FftRadix {
+  int n, r1, r2, r3;
+};
+constexpr FftRadix FFT_RADIX[] = {{3, 3, 1, 1},    {24, 6, 4, 1},   {36, 6, 6, 1},   {48, 6, 8, 1},   {72, 12, 6, 1},
+                                  {96, 12, 8, 1},  {144, 12, 12, 1}, {192, 12, 16, 1}, {288, 6, 6, 8},  {384, 6, 8, 8},
+                                  {576, 6, 8, 12}, {768, 12, 8, 8}, {1152, 12, 8, 12}, {1536, 12, 8, 16}};
 constexpr int NWB = 18;  // work-buffer slots: 12 + 6 transform inputs at most
 
 // Tables of the chunked y solves (lmc_ychunk.cuh), rows padded with zeros to
@@ -36,9 +44,7 @@ struct Dev {
               // (1 inverse z, 2 x stage, 4 direct z)
   int my, mgalx, mgalz, nkx, mz, nz1, nmode;
   int lpm, base, extra, C;  // y-chunking of a pencil over the lanes of a warp
-  int zb_x, kb_z;           // lines per block of the x / z transform kernels
   int smem_limit;           // opt-in shared memory per block of the device (bytes)
-  int xstg;                 // 1: the x stage stages its input rows where they fit (LMC_XSTG=0: never)
   // Slab blocks (lmc_step_split; the whole domain otherwise): the z
   // transforms cover kx planes zp0 .. zp0+zkn-1 with z-physical rows of zkn
   // values; the x stage covers its tiles xt0 .. xt0+xnt-1 (xnt 0: all), whose
@@ -75,7 +81,7 @@ struct Dev {
   // derivatives
   const double *r_dt12, *r_p1L, *r_p1U, *r_fmap, *r_ebot, *r_etop;
   const double *kx, *kz;  // wavenumber per kx plane / kz index
-  const double2 *twx, *twz;  // exp(-2 pi i e / N) for the x / z transform lengths
+  const double2 *twx, *twz;  // twiddles of the passes of the x / z transforms (fft_twiddles)
   const float2 *twxf, *twzf;  // the same in FP32 (mixed form)
   // state
   double2 *vor, *phi, *psi, *scal, *Rom, *Rphi;
@@ -146,9 +152,25 @@ struct Stats {
 };
 constexpr int NSTAT = 33;
 constexpr int XGRP = 32;  // z-tile groups of the physical-space sums
-// warps of an x-stage block at most: the mixed form's partial-sum slots
-// (Dev::mpart) hold one value per (z tile, warp)
-constexpr int XW_MAX = 9;
+// Threads of an x-stage block by transform length (f32: FP32 butterflies), and
+// the blocks per SM that its registers are sized for.  Where they were
+// measured, ms per step with the scalar and mu unless noted: 1152 FP32 256
+// threads 18.4 (320: 23.2 and 384: 20.3, the registers spill), FP64 384
+// threads 14.0 (512: 14.6, 576: 15.6); 384 FP32 128 threads 7.4 (192: 8.1,
+// 256: 9.7), FP64 192 threads 10.3 (128: 11.6, 256: 12.0); 288 FP64 without
+// them 160 threads 2.00 (192: 2.10, 256: 2.32); 144 FP32 without them six
+// blocks 0.54 (four: 0.57).
+// The mixed form's partial-sum slots (Dev::mpart) hold one value per (z tile,
+// warp).
+__host__ __device__ constexpr int x_block(int n, bool f32) {
+  return n == 1536 ? 384 : n == 1152 ? (f32 ? 256 : 384) : n == 768 ? (f32 ? 192 : 384) : n == 576 ? 288
+       : n == 384 ? (f32 ? 128 : 192) : n == 288 ? (f32 ? 128 : 160) : 128;
+}
+__host__ __device__ constexpr int x_minb(int n, bool f32) {
+  return n == 1536 ? 1 : n == 1152 ? (f32 ? 2 : 1) : n == 768 ? (f32 ? 3 : 1) : n == 576 ? 2
+       : n == 384 ? (f32 ? 4 : 3) : n == 288 ? 4 : f32 ? 6 : 4;
+}
+
 enum {
   ST_UM = 0, ST_VM, ST_WM, ST_RUM, ST_RVM, ST_RWM, ST_TM, ST_W1M, ST_W2M, ST_W3M, ST_THEM,
   ST_UP, ST_VP, ST_WP, ST_UVR, ST_UWR, ST_VWR, ST_W1P, ST_W2P, ST_W3P, ST_TP, ST_EP,
@@ -172,6 +194,15 @@ enum { OU = 0, OV, OW, ORUU, ORVV, ORWW, ORUV, ORUW, ORVW, ODRHO, ODT, ODZ };
 __host__ __device__ inline int vbase(const Dev &d) { return d.scalar ? 12 : 8; }
 __host__ __device__ inline int n_in(const Dev &d) { return vbase(d) + (d.visc ? 6 : 0); }
 __host__ __device__ inline int n_out(const Dev &d) { return d.scalar ? 12 : 11; }
+// The inverse z transforms skip the inputs that are an x derivative of
+// another: dT/dx (4) and, with the variable viscosity, d(rho u)/dx (vbase);
+// i kx does not depend on z, so the x stage forms them from T (7) and rho u
+// (0).  n_zin: the inputs transformed, in_field: the i-th of them.
+__host__ __device__ inline int n_zin(const Dev &d) { return n_in(d) - 1 - (d.visc ? 1 : 0); }
+__host__ __device__ inline int in_field(const Dev &d, int i) {
+  const int f = i < 4 ? i : i + 1;
+  return d.visc && f >= vbase(d) ? f + 1 : f;
+}
 // spectral and z-physical work buffers a case allocates
 __host__ __device__ inline int n_sbuf(const Dev &d) { return d.visc ? SB_G23 + 1 : n_out(d); }
 __host__ __device__ inline int n_zbuf(const Dev &d) { return n_in(d) > n_out(d) ? n_in(d) : n_out(d); }
@@ -222,8 +253,8 @@ void launch_xprep(const Dev &d, cudaStream_t s);
 void launch_xexport(const Dev &d, const int *jrow, int nplanes, int nf, double *out, cudaStream_t s);
 // mode 1 (2014 variant): the d(rho) round trip of T and Delta T; mode 2
 // (export, FP64): the inputs in slots xslot(f), rows in natural z order;
-// f0, nf: only inputs f0 .. f0+nf-1 (nf <= 0: all)
-void launch_zinv(const Dev &d, cudaStream_t s, int mode = 0, int f0 = 0, int nf = 0);
+// i0, n: only the transformed inputs in_field(i0) .. (n <= 0: all; mode 0)
+void launch_zinv(const Dev &d, cudaStream_t s, int mode = 0, int i0 = 0, int n = 0);
 void launch_xdrho(const Dev &d, cudaStream_t s);
 void launch_xphys(const Dev &d, int rk, int do_cfl, int do_diag, cudaStream_t s);
 void launch_zfwd(const Dev &d, cudaStream_t s, int mode = 0);
