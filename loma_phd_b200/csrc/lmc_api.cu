@@ -111,8 +111,9 @@ int dupload(lmc_handle *h, const T **p, const std::vector<T> &v) {
 }
 
 // Twiddles of the passes of a transform of length n (Fft in lmc_device.cuh):
-// exp(-2 pi i m k / n) at [k M + m], k < r1, m < M = r2 r3, then
-// exp(-2 pi i m k / M) at [n + k r3 + m], k < r2, m < r3.  C: double2 or float2
+// exp(-2 pi i m k / n) at [k M + m], k < r1, m < M = r2 r3; then
+// exp(-2 pi i m k / M) at [n + k r3 + m], k < r2, m < r3; then the direct
+// transform's.  C: double2 or float2
 template <typename C>
 std::vector<C> fft_twiddles(int n) {
   lmc::FftRadix f{n, n, 1, 1};
@@ -131,6 +132,10 @@ std::vector<C> fft_twiddles(int n) {
     for (int m = 0; m < M; m++) put((long long)k * m, n);
   for (int k = 0; k < f.r2; k++)
     for (int m = 0; m < f.r3; m++) put((long long)k * m, M);
+  // of the direct transform's first twiddled pass, the tasks fastest
+  const int jn = f.r3 > 1 ? f.r3 : M, fs = f.r3 > 1 ? f.r2 : f.r1, len = f.r3 > 1 ? M : n;
+  for (int j = 0; j < jn; j++)
+    for (int k = 0; k < fs; k++) put((long long)j * k, len);
   return t;
 }
 

@@ -600,18 +600,26 @@ __device__ __forceinline__ void line_tasks(int nb, Fn &&fn) {
 // The inverse ("inv") takes natural order and leaves X[k1 + R1 k2 + R1 R2 k3]
 // at position (k1 R2 + k2) R3 + k3; the direct one ("fwd") is its transpose,
 // so the samples are never reordered.  Line b starts at sm + b*ld; position n
-// is stored at sk(n), one pad slot per run of the last pass, so that its
-// strided tasks hit different banks.  tw: exp(-2 pi i n k1 / N) at [k1 M + n],
-// M = R2 R3, then exp(-2 pi i n k2 / M) at [N + k2 R3 + n].
+// is stored at sk(n), one pad slot per P positions (a multiple of the run of
+// the last pass), so that its strided tasks hit different banks.
+// tw: exp(-2 pi i n k1 / N) at [k1 M + n], M = R2 R3; exp(-2 pi i n k2 / M) at
+// [N + k2 R3 + n]; and at FW the factors of the direct transform's first
+// twiddled pass, exp(-2 pi i j k / M) (two passes: / N) of task k at
+// [FW + j FS + k]: with the tasks fastest the 16-byte loads of eight lanes are
+// one line of the L1 instead of eight, which were a quarter of the L1's cycles
+// of the FP64 x stage.
 // T: the threads of the block.  Every pass ends with a barrier.
-template <int R1, int R2, int R3, typename CT = double2, int T = 1>
+__host__ __device__ constexpr int fft_run(int r1, int r2, int r3) { return r3 > 1 ? r3 : r2 > 1 ? r2 : r1; }
+template <int R1, int R2, int R3, typename CT = double2, int T = 1, int P = fft_run(R1, R2, R3)>
 struct Fft {
   static constexpr int N = R1 * R2 * R3, M = R2 * R3, Q = R1 / 3;
-  static constexpr int RUN = R3 > 1 ? R3 : R2 > 1 ? R2 : N;
-  static constexpr int LD = N + (RUN < N ? N / RUN : 0);
+  static constexpr int RUN = fft_run(R1, R2, R3), PR = P / RUN;  // runs per pad slot
+  static constexpr int LD = N + (P < N ? N / P : 0);
+  static constexpr int FW = N + M, FS = R3 > 1 ? R2 : R1;
   static_assert(R1 % 3 == 0, "the 3/2-rule gap must be whole sample rows of the first pass");
-  __device__ static __forceinline__ int sk(int n) { return RUN < N ? n + n / RUN : n; }
-  static constexpr int SM = M + (RUN < N ? M / RUN : 0);  // sk(k M + n) = k SM + sk(n)
+  static_assert(P % RUN == 0 && (P == RUN || M % P == 0), "a pad slot follows whole runs");
+  __device__ static __forceinline__ int sk(int n) { return P < N ? n + n / P : n; }
+  static constexpr int SM = M + (P < N ? M / P : 0);  // sk(k M + n) = k SM + sk(n)
   // natural index of the sample at position n
   __device__ static __forceinline__ int nat(int n) {
     return n / M + R1 * ((n / R3) % R2) + R1 * R2 * (n % R3);
@@ -620,6 +628,16 @@ struct Fft {
   __device__ static __forceinline__ CT twd(const CT *__restrict__ tw, int e) {
     const CT w = __ldg(tw + e);
     return SIGN > 0 ? cconj(w) : w;
+  }
+
+  // slot of sample j of a second-pass task, from its first
+  __host__ __device__ static constexpr int at2(int j) { return R3 > 1 ? j * R3 + j / PR : j; }
+  // The k1 of the second-pass tasks in the order of the lanes.  FP32, runs of
+  // eight padded in pairs: lines k1 and k1 + 2 are eight banks apart, k1 and
+  // k1 + 1 four, so that the two of a half warp are two apart.
+  __device__ static __forceinline__ int lane_k1(int k) {
+    if constexpr (RUN == 8 && PR == 2 && SM % 8 == 4) return k < R1 / 4 * 4 ? (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1) : k;
+    else return k;
   }
 
   // first pass of the inverse: mk(b, n1) gives the reader of task n1 of line b,
@@ -649,19 +667,18 @@ struct Fft {
   __device__ static __forceinline__ void inv_p2(CT *sm, int nb, int ld, const CT *__restrict__ tw) {
     if constexpr (R2 > 1) {
       line_tasks<R1 * R3, T>(nb, [&](int b, int q) {
-        const int k1 = q / R3, n2 = q - k1 * R3;
+        const int k1 = lane_k1(q / R3), n2 = q % R3;
         CT *p = sm + (size_t)b * ld + k1 * SM + n2;
-        constexpr int ST = R3 > 1 ? R3 + 1 : 1;  // sk(R3)
         const CT *t = tw + N + n2;
         CT x[R2];
 #pragma unroll
-        for (int j = 0; j < R2; j++) x[j] = p[j * ST];
+        for (int j = 0; j < R2; j++) x[j] = p[at2(j)];
         rdft<R2, SIGN>(x);
 #pragma unroll
         for (int k = 0; k < R2; k++) {
           CT v = x[k];
           if (k > 0 && R3 > 1) v = cmul(v, twd<SIGN>(t, k * R3));
-          p[k * ST] = v;
+          p[at2(k)] = v;
         }
       });
       __syncthreads();
@@ -672,7 +689,7 @@ struct Fft {
   __device__ static __forceinline__ void inv_p3(CT *sm, int nb, int ld) {
     if constexpr (R3 > 1) {
       line_tasks<R1 * R2, T>(nb, [&](int b, int q) {
-        CT *p = sm + (size_t)b * ld + q * (R3 + 1);
+        CT *p = sm + (size_t)b * ld + q * R3 + q / PR;
         CT x[R3];
 #pragma unroll
         for (int j = 0; j < R3; j++) x[j] = p[j];
@@ -688,15 +705,14 @@ struct Fft {
   __device__ static __forceinline__ void fwd_p3(CT *sm, int nb, int ld, const CT *__restrict__ tw) {
     if constexpr (R3 > 1) {
       line_tasks<R1 * R2, T>(nb, [&](int b, int q) {
-        const int k2 = q % R2;
-        CT *p = sm + (size_t)b * ld + q * (R3 + 1);
-        const CT *t = tw + N + k2 * R3;
+        CT *p = sm + (size_t)b * ld + q * R3 + q / PR;
+        const CT *t = tw + FW + q % FS;
         CT x[R3];
 #pragma unroll
         for (int j = 0; j < R3; j++) x[j] = p[j];
         rdft<R3, SIGN>(x);
 #pragma unroll
-        for (int j = 0; j < R3; j++) p[j] = (j > 0) ? cmul(x[j], twd<SIGN>(t, j)) : x[j];
+        for (int j = 0; j < R3; j++) p[j] = (j > 0) ? cmul(x[j], twd<SIGN>(t, j * FS)) : x[j];
       });
       __syncthreads();
     }
@@ -705,16 +721,15 @@ struct Fft {
   __device__ static __forceinline__ void fwd_p2(CT *sm, int nb, int ld, const CT *__restrict__ tw) {
     if constexpr (R2 > 1) {
       line_tasks<R1 * R3, T>(nb, [&](int b, int q) {
-        const int k1 = q / R3, n2 = q - k1 * R3;
+        const int k1 = lane_k1(q / R3), n2 = q % R3;
         CT *p = sm + (size_t)b * ld + k1 * SM + n2;
-        constexpr int ST = R3 > 1 ? R3 + 1 : 1;
-        const CT *t = tw + k1 * M + n2;
+        const CT *t = R3 > 1 ? tw + k1 * M + n2 : tw + FW + k1;
         CT x[R2];
 #pragma unroll
-        for (int j = 0; j < R2; j++) x[j] = p[j * ST];
+        for (int j = 0; j < R2; j++) x[j] = p[at2(j)];
         rdft<R2, SIGN>(x);
 #pragma unroll
-        for (int j = 0; j < R2; j++) p[j * ST] = cmul(x[j], twd<SIGN>(t, j * R3));
+        for (int j = 0; j < R2; j++) p[at2(j)] = (R3 > 1 || j > 0) ? cmul(x[j], twd<SIGN>(t, j * (R3 > 1 ? R3 : FS))) : x[j];
       });
       __syncthreads();
     }

@@ -32,6 +32,26 @@ using namespace lmcd;
 namespace lmc {
 namespace LMC_FFT_NS {
 
+// The transforms of the x stage: a line is padded in whole bank rows (128 bytes
+// of samples), so that consecutive samples, which the first and the last pass
+// and the pointwise loop take, never share a bank, and the strided tasks of the
+// other passes do not either (FP32: but a third of the second pass's at 384
+// points, and that pass's at 288, 576 and 1152).  One slot per run left FP32
+// pairs of runs and FP64 runs of twelve in conflict.  With the twiddles of the
+// direct transforms in the order of the tasks (Fft) the x stage, which the L1
+// bounds, takes per step 9.14 ms after 10.23 (256 x 257 x 256, FP64, mu,
+// scalar), 12.56 after 13.97 (768 x 33), 1.70 after 2.00 (192 x 193 x 128);
+// FP32 17.6 after 18.3 (768 x 65).
+constexpr int x_pad(int r1, int r2, int r3, int un) {
+  const int run = fft_run(r1, r2, r3);
+  int p = run;
+  if (r3 > 1)
+    while (p % un) p += run;
+  return p;
+}
+template <int R1, int R2, int R3, typename CT, int T = 1>
+using XFft = Fft<R1, R2, R3, CT, T, x_pad(R1, R2, R3, 128 / (int)sizeof(CT))>;
+
 // Geometry of the x stage: z lines per tile, threads of a block, and the
 // blocks per SM that the registers are sized for.
 template <int R1, int R2, int R3>
@@ -202,9 +222,9 @@ __global__ void __launch_bounds__(ZGeo<R1, R2, R3, CT>::ZF, ZGeo<R1, R2, R3, CT>
     rdft<RL, -1>(x);
     CT *p = W + il * LD + (RL > 1 ? q * (RL + 1) : q);
     // twiddles: of the second pass after a third one, else of the first
-    const int e = R3 > 1 ? N + (q % R2) * R3 : q * M;
+    const int e = F::FW + q % F::FS;
 #pragma unroll
-    for (int j = 0; j < RL; j++) p[j] = (RL > 1 && j > 0) ? cmul(x[j], F::template twd<-1>(tw, e + j)) : x[j];
+    for (int j = 0; j < RL; j++) p[j] = (RL > 1 && j > 0) ? cmul(x[j], F::template twd<-1>(tw, e + j * F::FS)) : x[j];
   }
   __syncthreads();
   if constexpr (R3 > 1) F::template fwd_p2<-1>(W, nb, LD, tw);
@@ -242,7 +262,7 @@ __device__ __forceinline__ CT x_pack(CT a, CT c, int n, bool up) {
 // samples k and N - k of each other, and writes the retained kx of A and B.
 template <int R1, int R2, int R3, int T, typename CT, typename ST, typename AB>
 __device__ __forceinline__ void x_out(const Dev &d, const CT *sm, int nl, size_t gt, int nzb, AB &&ab) {
-  using F = Fft<R1, R2, R3, CT>;
+  using F = XFft<R1, R2, R3, CT>;
   using G = Geo<R1, R2, R3>;
   using Re = typename CReal<CT>::R;
   constexpr int N = F::N, M = F::M, Q = F::Q, ZB = G::ZB;
@@ -306,7 +326,7 @@ __global__ void __launch_bounds__(XGeo<R1, R2, R3, sizeof(CT) == sizeof(float2)>
                                   XGeo<R1, R2, R3, sizeof(CT) == sizeof(float2)>::MINB)
     k_xphys(Dev d, int rk, int do_cfl, int do_diag, int ntiles) {
   constexpr int XT = XGeo<R1, R2, R3, sizeof(CT) == sizeof(float2)>::XT;
-  using F = Fft<R1, R2, R3, CT, XT>;
+  using F = XFft<R1, R2, R3, CT, XT>;
   using G = Geo<R1, R2, R3>;
   using Re = typename CReal<CT>::R;
   constexpr int N = F::N, ZB = G::ZB, LD = G::LD;
@@ -586,7 +606,7 @@ __host__ __device__ constexpr int x_threads(int n) { return n >= 576 ? 256 : 128
 // a padding line)
 template <int R1, int R2, int R3, typename CT, typename ST, typename R>
 __device__ __forceinline__ void x_inverse(const Dev &d, CT *W, int nb, R &&rows) {
-  using F = Fft<R1, R2, R3, CT, x_threads(R1 * R2 * R3)>;
+  using F = XFft<R1, R2, R3, CT, x_threads(R1 * R2 * R3)>;
   constexpr int LD = Geo<R1, R2, R3>::LD;
   F::template inv_p1<+1>(W, nb, LD, wtwx<CT>(d), [&](int b, int n1) {
     const ST *A = nullptr, *B = nullptr;
@@ -609,7 +629,7 @@ __device__ __forceinline__ void x_inverse(const Dev &d, CT *W, int nb, R &&rows)
 template <int R1, int R2, int R3>
 __global__ void __launch_bounds__(x_threads(R1 *R2 *R3)) k_xexport(Dev d, const int *jrow, int nplanes, int nf,
                                                                   double *out) {
-  using F = Fft<R1, R2, R3, double2>;
+  using F = XFft<R1, R2, R3, double2>;
   using G = Geo<R1, R2, R3>;
   constexpr int N = F::N, ZB = G::ZB, LD = G::LD;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -645,7 +665,7 @@ __global__ void __launch_bounds__(x_threads(R1 *R2 *R3)) k_xexport(Dev d, const 
 // complex line per (y, z), the result leaves in z-physical buffer 0.
 template <int R1, int R2, int R3>
 __global__ void __launch_bounds__(x_threads(R1 *R2 *R3)) k_xdrho(Dev d) {
-  using F = Fft<R1, R2, R3, double2, x_threads(R1 * R2 * R3)>;
+  using F = XFft<R1, R2, R3, double2, x_threads(R1 * R2 * R3)>;
   using G = Geo<R1, R2, R3>;
   constexpr int N = F::N, ZB = G::ZB, LD = G::LD;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -683,7 +703,7 @@ __global__ void __launch_bounds__(x_threads(R1 *R2 *R3)) k_xdrho(Dev d) {
 // row in order, so the sums are reproducible.
 template <int R1, int R2, int R3, typename CT, typename ST>
 __global__ void __launch_bounds__(x_threads(R1 *R2 *R3)) k_xstats(Dev d, Stats st, int ngrp) {
-  using F = Fft<R1, R2, R3, CT>;
+  using F = XFft<R1, R2, R3, CT>;
   using G = Geo<R1, R2, R3>;
   constexpr int N = F::N, ZB = G::ZB, LD = G::LD, NW = x_threads(N) / 32;
   extern __shared__ __align__(16) unsigned char smraw[];
