@@ -184,12 +184,12 @@ constexpr int FEW_MODES = 8 * 2 * 148;
 
 // Blocks of the sweeps along y (lmc_ysweep.cuh), which take over from the
 // chunked kernels (not in the 2014 variant) for grids with many modes, where
-// the sweeps fill the device (an FP64 step of 12,192 modes x 193 takes 7.4 ms
-// with the chunks and 7.6 with the sweeps, one of 8,128 x 129 3.35 and
-// 4.26 ms; 32,640 x 257 with mu = T^0.7, the scalar and float2 buffers 25.7
-// and 20.6), and for short pencils, which a chunk or three hold (with the
-// scalar and mu, 3,040 to 12,192 modes: the sweeps take 0.79 to 0.86 of the
-// chunks' step at 18 rows, 0.90 to 0.93 at 24 and 0.99 to 1.09 at 33).
+// the sweeps fill the device (an FP64 step of 12,192 modes x 193 takes 5.3 ms
+// with the chunks and 5.8 with the sweeps, one of 8,128 x 129 2.5 and
+// 3.4 ms; 32,640 x 257 with mu = T^0.7, the scalar and float2 buffers 21.1
+// and 17.2), and for short pencils, which a chunk or three hold (with the
+// scalar and mu, 3,040 to 12,192 modes: the sweeps take 0.81 to 0.92 of the
+// chunks' step at 18 rows, 0.90 to 1.03 at 24 and 1.03 to 1.24 at 33).
 int sweep_blocks(const lmc::Grid &g, int variant) {
   const bool force = std::getenv("LMC_YPATH") != nullptr;
   if (variant || !(many_modes(g.nmode) || (!force && g.my <= 28 && g.nmode > FEW_MODES))) return 0;
@@ -204,11 +204,12 @@ size_t sweep_scratch(int ysb, int q, const lmc::Grid &g) {
 // Geometry of the chunked y kernels (lmc_ychunk.cuh): rows per chunk and
 // modes per block.  Short chunks where the blocks of eight modes are at most
 // two per SM, so that the length of one block's chain is what counts (2,016
-// modes x 129, FP64: 1.32 ms per step against 1.41 with nine rows; 256 x
-// 257: 0.80 against 0.88); above that nine rows, which load fewer
+// modes x 129, FP64: 0.93 ms per step against 1.04 with nine rows; 256 x
+// 257: 0.69 against 0.79); above that nine rows, which load fewer
 // coefficients per row, and as many modes per block as 512 threads allow
-// (4,560 x 129, float2 buffers: 1.50 against 1.56 ms; 12,192 x 193, FP64:
-// 7.43 with 16 modes, 7.54 with 8, 7.87 with five rows).
+// (4,560 x 129, float2 buffers: 1.29 ms, 1.41 with 8 modes, 1.35 with five
+// rows; 12,192 x 193, FP64: 5.29 with 16 modes, 5.65 with 8, 5.79 with five
+// rows).
 void y_geometry(lmc::Dev &d, const lmc::Grid &g) {
   d.ysb = sweep_blocks(g, d.variant);
   const bool few = !many_modes(g.nmode) && g.nmode <= FEW_MODES;
@@ -435,16 +436,29 @@ int lmc_create(const lmc_params *p, const double *y, lmc_handle **out) {
     lmc_destroy(h);
     return rc;
   }
-  lmc::YChunk &q = d.ct;
-  if ((rc = dupload(h, &q.fw1, ct.fw1)) || (rc = dupload(h, &q.hl1, ct.hl1)) || (rc = dupload(h, &q.bw1, ct.bw1)) ||
-      (rc = dupload(h, &q.hu1, ct.hu1)) || (rc = dupload(h, &q.fw2, ct.fw2)) || (rc = dupload(h, &q.hl2, ct.hl2)) ||
-      (rc = dupload(h, &q.bw2, ct.bw2)) || (rc = dupload(h, &q.hu2, ct.hu2)) || (rc = dupload(h, &q.fwp, ct.fwp)) ||
-      (rc = dupload(h, &q.m1L, ct.m1L)) || (rc = dupload(h, &q.q1L, ct.q1L)) || (rc = dupload(h, &q.g1L, ct.g1L)) ||
-      (rc = dupload(h, &q.m1U, ct.m1U)) || (rc = dupload(h, &q.q1U, ct.q1U)) || (rc = dupload(h, &q.g1U, ct.g1U)) ||
-      (rc = dupload(h, &q.m2L, ct.m2L)) || (rc = dupload(h, &q.q2L, ct.q2L)) || (rc = dupload(h, &q.g2L, ct.g2L)) ||
-      (rc = dupload(h, &q.m2U, ct.m2U)) || (rc = dupload(h, &q.q2U, ct.q2U)) || (rc = dupload(h, &q.g2U, ct.g2U))) {
-    lmc_destroy(h);
-    return rc;
+  {
+    lmc::YChunk &q = d.ct;
+    const std::pair<const double **, const std::vector<double> *> part[] = {
+        {&q.fw1, &ct.fw1}, {&q.hl1, &ct.hl1}, {&q.bw1, &ct.bw1}, {&q.hu1, &ct.hu1}, {&q.m1L, &ct.m1L},
+        {&q.q1L, &ct.q1L}, {&q.g1L, &ct.g1L}, {&q.m1U, &ct.m1U}, {&q.q1U, &ct.q1U}, {&q.g1U, &ct.g1U}, {&q.fw2, &ct.fw2},
+        {&q.hl2, &ct.hl2}, {&q.bw2, &ct.bw2}, {&q.hu2, &ct.hu2}, {&q.m2L, &ct.m2L}, {&q.q2L, &ct.q2L}, {&q.g2L, &ct.g2L},
+        {&q.m2U, &ct.m2U}, {&q.q2U, &ct.q2U}, {&q.g2U, &ct.g2U}};
+    std::vector<double> all;
+    std::vector<size_t> at;
+    for (const auto &p : part) {
+      at.push_back(all.size());
+      all.insert(all.end(), p.second->begin(), p.second->end());
+      all.resize((all.size() + 1) / 2 * 2, 0.0);  // 16-byte rows
+    }
+    const double *run = nullptr;
+    if ((rc = dupload(h, &run, all)) || (rc = dupload(h, &q.fwp, ct.fwp))) {
+      lmc_destroy(h);
+      return rc;
+    }
+    for (size_t i = 0; i < at.size(); i++) *part[i].first = run + at[i];
+    q.n1 = (int)at[10];
+    q.n2 = (int)all.size() - q.n1;
+    q.sm = 0;
   }
   // the per-mode tables are on the device now
   h->pt = lmc::PoissonTables();

@@ -29,6 +29,9 @@ constexpr int NWB = 18;  // work-buffer slots: 12 + 6 transform inputs at most
 struct YChunk {
   const double *fw1, *hl1, *bw1, *hu1, *fw2, *hl2, *bw2, *hu2, *fwp;
   const double *m1L, *q1L, *g1L, *m1U, *q1U, *g1U, *m2L, *q2L, *g2L, *m2U, *q2U, *g2U;
+  // the tables of d/dy are one run of n1 values from fw1 on, those of d2/dy2
+  // the next n2; sm: the launch has room for them in shared memory
+  int n1, n2, sm;
 };
 
 // Device-side view of one case.

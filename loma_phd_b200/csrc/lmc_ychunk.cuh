@@ -21,7 +21,8 @@
 // four lanes per pencil walk a quarter of the chunks each, join their ends
 // by shuffles, and every chunk adds Q S_group itself.  For the operators
 // that do not depend on the mode the tables M, Q, H come from the host
-// (build_chunk_tables); for the per-mode Poisson LUs they are formed by two
+// (build_chunk_tables) and are copied to shared memory where they fit (go);
+// for the per-mode Poisson LUs they are formed by two
 // real recurrences beside the particular one.
 // Rows past my (the last chunk's padding) have zero coefficients.
 //
@@ -29,6 +30,10 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <type_traits>
+
+#include "lmc_async.cuh"
 #include "lmc_ylaunch.h"
 
 namespace lmc {
@@ -73,13 +78,50 @@ struct Sm {
   double2 *P;  // [F][nc][3][MB]
   double2 *G;  // [F][4][3][MB]
   double *Q;   // [nc][4][MB]
-  __device__ __forceinline__ Sm(int nc, int F, unsigned char *raw) {
+  const double *tb, *gb;  // the tables of d/dy and d2/dy2: where they are read, and in global memory
+  bool two;               // d2/dy2's as well
+  // TAB: the kernel uses those of d/dy (1), of both (2) or none
+  template <int TAB>
+  __device__ __forceinline__ void init(const Dev &d, int nc, int F, bool poisson, unsigned char *raw) {
     E = (double2 *)raw;
     P = E + F * nc * 6 * MB;
     G = P + F * nc * 3 * MB;
     Q = (double *)(G + F * 12 * MB);
+    tb = gb = d.ct.fw1;
+    two = TAB > 1;
+    if (TAB > 0 && d.ct.sm) {  // on their way while the first rows are read
+      double *t = (double *)(raw + bytes(nc, F, poisson));
+      for (int i = 2 * threadIdx.x; i < d.ct.n1; i += 2 * blockDim.x) cp16(t + i, gb + i);
+      cp_commit();
+      if (TAB > 1)  // a group of its own
+        for (int i = d.ct.n1 + 2 * threadIdx.x; i < d.ct.n1 + d.ct.n2; i += 2 * blockDim.x) cp16(t + i, gb + i);
+      cp_commit();
+      tb = t;
+    }
   }
-  static size_t bytes(int nc, int F, bool poisson) {
+  // before the first use of the tables of d/dy, and of d2/dy2
+  __device__ __forceinline__ void tables1() const {
+    if (tb != gb) {
+      cp_wait<1>();
+      __syncthreads();
+    }
+  }
+  __device__ __forceinline__ void tables2() const {
+    if (two && tb != gb) {
+      cp_wait<0>();
+      __syncthreads();
+    }
+  }
+  __device__ __forceinline__ const double *t(const double *p) const { return tb + (p - gb); }
+  __device__ __forceinline__ const double *t2(const double *p) const { return two ? t(p) : p; }
+  template <int B>  // of the tables of d/dy (B = 3) or of d2/dy2 (2)
+  __device__ __forceinline__ double ld1(const double *p) const {
+    return B == 3 || two ? *p : __ldg(p);
+  }
+  __device__ __forceinline__ double2 ld2(const double *p) const {
+    return two ? *(const double2 *)p : __ldg((const double2 *)p);
+  }
+  __host__ __device__ static size_t bytes(int nc, int F, bool poisson) {
     return sizeof(double2) * ((size_t)F * nc * 9 * MB + F * 12 * MB) + (poisson ? sizeof(double) * nc * 4 * MB : 0);
   }
 };
@@ -90,6 +132,7 @@ __device__ __forceinline__ double2 fms2(double2 s, double k, double2 v) {
 __device__ __forceinline__ double2 fma2(double2 s, double k, double2 v) {
   return make_double2(fma(k, v.x, s.x), fma(k, v.y, s.y));
 }
+__device__ __forceinline__ double2 ld2(const double *p) { return *(const double2 *)p; }
 __device__ __forceinline__ double2 ldg2(const double *p) { return __ldg((const double2 *)p); }
 
 // the thread's rows of a field, and the same with three more rows on either
@@ -154,7 +197,7 @@ __device__ __forceinline__ void shfl_state(double2 (&t)[B], const double2 (&s)[B
     t[q] = make_double2(__shfl_sync(LMC_FULL, s[q].x, src), __shfl_sync(LMC_FULL, s[q].y, src));
 }
 template <int B, int MB, bool UP>
-__device__ __forceinline__ void scan_unit(int sub, int nc, double2 *P, double2 *G, const double *__restrict__ M,
+__device__ __forceinline__ void scan_unit(int sub, int nc, const Sm<MB> &S, double2 *P, double2 *G, const double *__restrict__ M,
                                           const double *__restrict__ GM) {
   const int lane = threadIdx.x & 31, g = lane & 3, ml = sub * 8 + (lane >> 2);
   const int gl = (nc + 3) >> 2, i0 = g * gl, i1 = min(nc, i0 + gl);
@@ -173,7 +216,7 @@ __device__ __forceinline__ void scan_unit(int sub, int nc, double2 *P, double2 *
 #pragma unroll
     for (int r = 0; r < B; r++)
 #pragma unroll
-      for (int q = 0; q < B; q++) n[r] = fma2(n[r], __ldg(mt + r * B + q), s[q]);
+      for (int q = 0; q < B; q++) n[r] = fma2(n[r], S.template ld1<B>(mt + r * B + q), s[q]);
 #pragma unroll
     for (int q = 0; q < B; q++) s[q] = n[q];
   }
@@ -185,7 +228,7 @@ __device__ __forceinline__ void scan_unit(int sub, int nc, double2 *P, double2 *
 #pragma unroll
       for (int r = 0; r < B; r++)
 #pragma unroll
-        for (int q = 0; q < B; q++) t[r] = fma2(t[r], __ldg(GM + (k * B + r) * B + q), e[q]);
+        for (int q = 0; q < B; q++) t[r] = fma2(t[r], S.template ld1<B>(GM + (k * B + r) * B + q), e[q]);
 #pragma unroll
       for (int q = 0; q < B; q++) e[q] = t[q];
     }
@@ -251,8 +294,8 @@ __device__ __forceinline__ void scans(const Dev &d, int nc, const Sm<MB> &S) {
     for (int u = w; u < (F1 + F2) * SUB; u += nw) {
       const int f = u / SUB, sub = u - f * SUB;
       double2 *P = S.P + (size_t)f * nc * 3 * MB, *G = S.G + f * 12 * MB;
-      if (f < F1) scan_unit<3, MB, UP>(sub, nc, P, G, UP ? q.m1U : q.m1L, UP ? q.g1U : q.g1L);
-      else scan_unit<2, MB, UP>(sub, nc, P, G, UP ? q.m2U : q.m2L, UP ? q.g2U : q.g2L);
+      if (f < F1) scan_unit<3, MB, UP>(sub, nc, S, P, G, S.t(UP ? q.m1U : q.m1L), S.t(UP ? q.g1U : q.g1L));
+      else scan_unit<2, MB, UP>(sub, nc, S, P, G, S.t2(UP ? q.m2U : q.m2L), S.t2(UP ? q.g2U : q.g2L));
     }
   __syncthreads();
 }
@@ -282,7 +325,7 @@ __device__ __forceinline__ void get_state(const Th<C, MB> &T, const Sm<MB> &S, i
   for (int r = 0; r < B; r++) {
     double2 v = p[r * MB];
 #pragma unroll
-    for (int q = 0; q < B; q++) v = fma2(v, __ldg(Q + (i * B + r) * B + q), e[q * MB]);
+    for (int q = 0; q < B; q++) v = fma2(v, S.template ld1<B>(Q + (i * B + r) * B + q), e[q * MB]);
     s[r] = v;
   }
 }
@@ -304,13 +347,13 @@ __device__ __forceinline__ void get_state_p(const Th<C, MB> &T, const Sm<MB> &S,
 template <int C, int MB>
 __device__ __forceinline__ void d1_fwd(const Dev &d, const Th<C, MB> &T, const Sm<MB> &S, int slot,
                                        const double2 (&u)[C + 6], double2 (&w)[C]) {
-  const double *r = d.ct.fw1 + (size_t)T.j0 * 10;
+  const double *r = S.t(d.ct.fw1) + (size_t)T.j0 * 10;
 #pragma unroll
   for (int t = 0; t < C; t++) {
     double k[10];
 #pragma unroll
     for (int q = 0; q < 5; q++) {
-      const double2 v = ldg2(r + t * 10 + 2 * q);
+      const double2 v = ld2(r + t * 10 + 2 * q);
       k[2 * q] = v.x;
       k[2 * q + 1] = v.y;
     }
@@ -329,11 +372,11 @@ template <int C, int MB, int F>
 __device__ __forceinline__ void d1_bwd(const Dev &d, const Th<C, MB> &T, const Sm<MB> &S, double2 (&w)[F][C]) {
   double2 s[F][3];
 #pragma unroll
-  for (int f = 0; f < F; f++) get_state<3, false>(T, S, f, d.ct.q1L, s[f]);
-  const double *hl = d.ct.hl1 + (size_t)T.j0 * 4, *bw = d.ct.bw1 + (size_t)T.j0 * 4;
+  for (int f = 0; f < F; f++) get_state<3, false>(T, S, f, S.t(d.ct.q1L), s[f]);
+  const double *hl = S.t(d.ct.hl1) + (size_t)T.j0 * 4, *bw = S.t(d.ct.bw1) + (size_t)T.j0 * 4;
 #pragma unroll
   for (int t = C - 1; t >= 0; t--) {
-    const double2 h0 = ldg2(hl + t * 4), h1 = ldg2(hl + t * 4 + 2), b0 = ldg2(bw + t * 4), b1 = ldg2(bw + t * 4 + 2);
+    const double2 h0 = ld2(hl + t * 4), h1 = ld2(hl + t * 4 + 2), b0 = ld2(bw + t * 4), b1 = ld2(bw + t * 4 + 2);
 #pragma unroll
     for (int f = 0; f < F; f++) {
       double2 a = fma2(fma2(fma2(w[f][t], h0.x, s[f][0]), h0.y, s[f][1]), h1.x, s[f][2]);
@@ -354,11 +397,11 @@ template <int C, int MB, int F>
 __device__ __forceinline__ void d1_end(const Dev &d, const Th<C, MB> &T, const Sm<MB> &S, double2 (&w)[F][C]) {
   double2 s[F][3];
 #pragma unroll
-  for (int f = 0; f < F; f++) get_state<3, true>(T, S, f, d.ct.q1U, s[f]);
-  const double *hu = d.ct.hu1 + (size_t)T.j0 * 4;
+  for (int f = 0; f < F; f++) get_state<3, true>(T, S, f, S.t(d.ct.q1U), s[f]);
+  const double *hu = S.t(d.ct.hu1) + (size_t)T.j0 * 4;
 #pragma unroll
   for (int t = 0; t < C; t++) {
-    const double2 h0 = ldg2(hu + t * 4), h1 = ldg2(hu + t * 4 + 2);
+    const double2 h0 = ld2(hu + t * 4), h1 = ld2(hu + t * 4 + 2);
 #pragma unroll
     for (int f = 0; f < F; f++)
       w[f][t] = cscale(h1.y, fma2(fma2(fma2(w[f][t], h0.x, s[f][0]), h0.y, s[f][1]), h1.x, s[f][2]));
@@ -381,13 +424,13 @@ __device__ __forceinline__ void d1_rest(const Dev &d, const Th<C, MB> &T, const 
 template <int C, int MB>
 __device__ __forceinline__ void d2_fwd(const Dev &d, const Th<C, MB> &T, const Sm<MB> &S, int slot, double kk,
                                        const double2 (&u)[C + 6], double2 (&w)[C]) {
-  const double *r = d.ct.fw2 + (size_t)T.j0 * 12;
+  const double *r = S.t2(d.ct.fw2) + (size_t)T.j0 * 12;
 #pragma unroll
   for (int t = 0; t < C; t++) {
     double k[12];
 #pragma unroll
     for (int q = 0; q < 6; q++) {
-      const double2 v = ldg2(r + t * 12 + 2 * q);
+      const double2 v = S.ld2(r + t * 12 + 2 * q);
       k[2 * q] = v.x;
       k[2 * q + 1] = v.y;
     }
@@ -404,11 +447,11 @@ __device__ __forceinline__ void d2_fwd(const Dev &d, const Th<C, MB> &T, const S
 template <int C, int MB>
 __device__ __forceinline__ void d2_bwd(const Dev &d, const Th<C, MB> &T, const Sm<MB> &S, int slot, double2 (&w)[C]) {
   double2 s[2];
-  get_state<2, false>(T, S, slot, d.ct.q2L, s);
-  const double *hl = d.ct.hl2 + (size_t)T.j0 * 2, *bw = d.ct.bw2 + (size_t)T.j0 * 4;
+  get_state<2, false>(T, S, slot, S.t2(d.ct.q2L), s);
+  const double *hl = S.t2(d.ct.hl2) + (size_t)T.j0 * 2, *bw = S.t2(d.ct.bw2) + (size_t)T.j0 * 4;
 #pragma unroll
   for (int t = C - 1; t >= 0; t--) {
-    const double2 h = ldg2(hl + t * 2), b0 = ldg2(bw + t * 4), b1 = ldg2(bw + t * 4 + 2);
+    const double2 h = S.ld2(hl + t * 2), b0 = S.ld2(bw + t * 4), b1 = S.ld2(bw + t * 4 + 2);
     double2 a = cscale(b0.x, fma2(fma2(w[t], h.x, s[0]), h.y, s[1]));
     if (t + 2 < C) a = fms2(a, b1.x, w[t + 2]);
     if (t + 1 < C) a = fms2(a, b0.y, w[t + 1]);
@@ -420,11 +463,11 @@ __device__ __forceinline__ void d2_bwd(const Dev &d, const Th<C, MB> &T, const S
 template <int C, int MB>
 __device__ __forceinline__ void d2_end(const Dev &d, const Th<C, MB> &T, const Sm<MB> &S, int slot, double2 (&w)[C]) {
   double2 s[2];
-  get_state<2, true>(T, S, slot, d.ct.q2U, s);
-  const double *hu = d.ct.hu2 + (size_t)T.j0 * 2;
+  get_state<2, true>(T, S, slot, S.t2(d.ct.q2U), s);
+  const double *hu = S.t2(d.ct.hu2) + (size_t)T.j0 * 2;
 #pragma unroll
   for (int t = 0; t < C; t++) {
-    const double2 h = ldg2(hu + t * 2);
+    const double2 h = S.ld2(hu + t * 2);
     w[t] = fma2(fma2(w[t], h.x, s[0]), h.y, s[1]);
   }
 }
@@ -511,17 +554,18 @@ __device__ __forceinline__ double2 mo00(const Dev &d, int o, int j) {
   return make_double2(d.mo_cur[(size_t)o * d.my + j] / ((double)d.mgalx * (double)d.mgalz), 0.0);
 }
 
-#define LMC_YC_PROLOGUE(F)                        \
+#define LMC_YC_PROLOGUE(F, POISSON, TAB)               \
   extern __shared__ __align__(16) unsigned char raw[]; \
-  const Th<C, MB> T(d);                           \
-  const Sm<MB> S(T.nc, F, raw);
+  const Th<C, MB> T(d);                                \
+  Sm<MB> S;                                            \
+  S.template init<TAB>(d, T.nc, F, POISSON, raw);
 
 // ----------------------------------------------------------------------
 // (1) Lapvdvhom: phi -> m_y, dm_y/dy (cross.f:329-335, 365-372)
 // ----------------------------------------------------------------------
 template <typename CT, int C, int MB>
 __global__ void __launch_bounds__(YC_TMAX, 1) c_lapv(Dev d) {
-  LMC_YC_PROLOGUE(1)
+  LMC_YC_PROLOGUE(1, true, 1)
   double2 x[1][C];
   {
     double2 u[C + 6];
@@ -532,6 +576,7 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_lapv(Dev d) {
       if (j == 0 || j == d.my - 1) u[t] = czero();
     }
     poisson(d, T, S, u, x[0]);
+    S.tables1();
   }
   store(T, wsb<CT>(d, SB_MY), x[0]);
   put_edges(T, S, 0, x[0]);
@@ -554,7 +599,7 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_lapv(Dev d) {
 // ----------------------------------------------------------------------
 template <typename CT, int C, int MB, bool V>
 __global__ void __launch_bounds__(YC_TMAX, 1) c_assemble(Dev d, int rk) {
-  LMC_YC_PROLOGUE(1)
+  LMC_YC_PROLOGUE(1, false, 1)
   const int my = d.my;
   const double dtxi = d.scal_d[0] * d.xi[rk];
   const double ta = (T.k2 != 0.0) ? T.kx / T.k2 : 0.0, tb = (T.k2 != 0.0) ? T.kz / T.k2 : 0.0;
@@ -567,6 +612,7 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_assemble(Dev d, int rk) {
   {
     double2 u[C + 6];
     rows_h(d, T, d.psi, u);
+    S.tables1();
     d1_fwd(d, T, S, 0, u, x[0]);
   }
   d1_rest(d, T, S, x);
@@ -638,9 +684,9 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_assemble(Dev d, int rk) {
 // values imposed (lomacte/cross.f:486-519).  Z: the passive scalar, treated
 // as T, its 00 mode held at scal_d[5], scal_d[6] (mi rows 6, 7).
 // ----------------------------------------------------------------------
-template <typename CT, int C, int MB, bool V, bool Z>
+template <typename CT, int C, int MB, bool V, bool Z, int TAB>
 __global__ void __launch_bounds__(YC_TMAX, 1) c_tder(Dev d) {
-  LMC_YC_PROLOGUE(2)
+  LMC_YC_PROLOGUE(2, false, TAB)
   const int my = d.my;
   const bool m00 = T.act && T.m == 0;
   double2 *const f = Z ? d.zsc : V ? d.Told : d.scal;
@@ -671,7 +717,9 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_tder(Dev d) {
       }
       store(T, wsb<CT>(d, Z ? SB_Z32 : SB_T32), v);
     }
+    S.tables1();
     d1_fwd(d, T, S, 0, u, a[0]);
+    S.tables2();
     d2_fwd(d, T, S, 1, T.k2, u, b);
   }
   d12_rest(d, T, S, a, b);
@@ -703,7 +751,7 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_tder(Dev d) {
 // ----------------------------------------------------------------------
 template <typename CT, int C, int MB>
 __global__ void __launch_bounds__(YC_TMAX, 1) c_sgrad(Dev d) {
-  LMC_YC_PROLOGUE(1)
+  LMC_YC_PROLOGUE(1, false, 1)
   double2 x[1][C];
   if constexpr (mixed<CT>()) {
     if (blockIdx.x == gridDim.x - 1) {
@@ -714,6 +762,7 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_sgrad(Dev d) {
         const int j = T.j0 + t - 3;
         u[t] = make_double2((j >= 0 && j < d.my) ? p[j] : 0.0, 0.0);
       }
+      S.tables1();
       d1_fwd(d, T, S, 0, u, x[0]);
       d1_rest(d, T, S, x);
       if (T.ml < 3) {
@@ -726,21 +775,22 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_sgrad(Dev d) {
     }
   }
   const CT *RU = wsb<CT>(d, SB_RU), *RV = wsb<CT>(d, SB_RV), *RW = wsb<CT>(d, SB_RW);
-  auto deriv = [&](const CT *f) {
+  auto deriv = [&](const CT *f, bool first) {
     double2 u[C + 6];
     rows_h(d, T, f, u);
+    if (first) S.tables1();
     d1_fwd(d, T, S, 0, u, x[0]);
     d1_rest(d, T, S, x);
   };
-  deriv(RV);
+  deriv(RV, true);
   store(T, wsb<CT>(d, SB_GYY), x[0]);
-  deriv(RU);
+  deriv(RU, false);
   double2 v[C];
   rows(T, RV, v);
 #pragma unroll
   for (int t = 0; t < C; t++) x[0][t] = cadd(x[0][t], cik(T.kx, v[t]));
   store(T, wsb<CT>(d, SB_G12), x[0]);
-  deriv(RW);
+  deriv(RW, false);
   rows(T, RV, v);
 #pragma unroll
   for (int t = 0; t < C; t++) x[0][t] = cadd(x[0][t], cik(T.kz, v[t]));
@@ -768,9 +818,9 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_sgrad(Dev d) {
 // N_i or curl goes through memory.  TU: T += Delta T as well (cross.f:
 // 619-627); grids with many modes leave that to c_tupd on the second stream.
 // ----------------------------------------------------------------------
-template <typename CT, int C, int MB, bool TU>
+template <typename CT, int C, int MB, bool TU, int TAB>
 __global__ void __launch_bounds__(YC_TMAX, 1) c_post(Dev d, int rk) {
-  LMC_YC_PROLOGUE(2)
+  LMC_YC_PROLOGUE(2, false, TAB)
   const double kx = T.kx, kz = T.kz, k2 = T.k2, dtg = d.scal_d[0] * d.gama[rk];
   const CT *U = wsb<CT>(d, OU), *V = wsb<CT>(d, OV), *W = wsb<CT>(d, OW);
   const CT *UU = wsb<CT>(d, ORUU), *VV = wsb<CT>(d, ORVV), *WW = wsb<CT>(d, ORWW);
@@ -793,11 +843,13 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_post(Dev d, int rk) {
     {
       double2 u[C + 6];
       comb(kx, UV, kz, VW, u);
+      S.tables1();
       d1_fwd(d, T, S, 0, u, x[0]);
       comb(kx, U, kz, W, u);
       d1_fwd(d, T, S, 1, u, x[1]);
     }
     d1_rest(d, T, S, x);
+    S.tables2();
 #pragma unroll
     for (int t = 0; t < C; t++) {
       if (t < T.n) {
@@ -929,7 +981,7 @@ __device__ __forceinline__ void neumann(const Dev &d, const Th<C, MB> &T, const 
 }
 template <typename CT, int C, int MB, bool V>
 __global__ void __launch_bounds__(YC_TMAX, 1) c_psi(Dev d, int rk) {
-  LMC_YC_PROLOGUE(1)
+  LMC_YC_PROLOGUE(1, true, 0)
   double2 x[C];
   {
     double2 u[C + 6];
@@ -949,11 +1001,13 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_psi(Dev d, int rk) {
 // 3 Lapvdvhom (out = v, out2 = dv/dy), 4 solvepsi
 template <int C, int MB>
 __global__ void __launch_bounds__(YC_TMAX, 1) c_op(Dev d, int op, const double2 *in, double2 *out, double2 *out2) {
-  LMC_YC_PROLOGUE(2)
+  LMC_YC_PROLOGUE(2, true, 2)
   double2 x[1][C], b[C];
   {
     double2 u[C + 6];
     rows_h(d, T, in, u);
+    S.tables1();
+    S.tables2();
     if (op <= 2) {
       d1_fwd(d, T, S, 0, u, x[0]);
       d2_fwd(d, T, S, 1, 0.0, u, b);
@@ -984,74 +1038,115 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_op(Dev d, int op, const double2 
 }  // namespace ych
 
 namespace ych {
-// one block per MB modes (and `extra`), shared memory for F pencils
+// Blocks from which c_tder and c_post take the tables of d2/dy2 from shared
+// memory as well as those of d/dy: with several waves of blocks they are out
+// of the L1 each time (12,192 modes x 193, FP64, five waves: 5.29 ms per step
+// against 5.43); with one or two a block waits for more bytes than it saves
+// (2,016 x 129: 0.93 against 0.98; 4,560 x 129 1.29 against 1.32).
+template <int MB>
+bool many_waves(const Dev &d) {
+  return (d.nmode + MB - 1) / MB > 4 * 148;
+}
+// One block per MB modes (and `extra`), shared memory for F pencils and for
+// the tables of d/dy (tabs 1) and of d2/dy2 (tabs 2), which every block reads
+// several times: from global memory they come out of the L2 with each pass,
+// as the pencils' rows push them out of the L1 (c_post, 12,192 x 193: 16 of
+// 25 cycles between a warp's instructions were waits for loads).  They stay
+// there where shared memory has no room for them or would hold fewer blocks
+// per SM than the registers do.  24 x 25 x 24: 0.230 ms per step after 0.240;
+// 64 x 129 x 64 with the scalar and mu 0.93 after 1.00; 96 x 129 x 96, float2
+// buffers, 1.29 after 1.33; 192 x 193 x 128 5.29 after 5.60.
 template <int MB, typename K, typename... A>
-void go(K k, const Dev &d, int F, bool poisson, int extra, cudaStream_t s, A... a) {
-  const unsigned g = (unsigned)((d.nmode + MB - 1) / MB + extra);
-  k<<<g, d.ync * MB, Sm<MB>::bytes(d.ync, F, poisson), s>>>(a...);
+void go(K k, const Dev &d, int F, bool poisson, int tabs, int extra, cudaStream_t s, A... a) {
+  const int g = (d.nmode + MB - 1) / MB + extra, nt = d.ync * MB;
+  const size_t base = Sm<MB>::bytes(d.ync, F, poisson);
+  const size_t tab = sizeof(double) * (tabs == 2 ? d.ct.n1 + d.ct.n2 : tabs == 1 ? d.ct.n1 : 0);
+  const size_t sm = 228 * 1024, res = 1024;                // shared memory of an SM, and what each block reserves of it
+  size_t per = 64 / ((nt + 31) / 32 * 4);  // blocks by registers (128 each)
+  per = std::min(std::max<size_t>(per, 1), std::min<size_t>(sm / (base + res), (g + 147) / 148));
+  Dev e = d;
+  e.ct.sm = tab > 0 && base + tab <= (size_t)d.smem_limit && per * (base + tab + res) <= sm;
+  k<<<g, nt, base + (e.ct.sm ? tab : 0), s>>>(e, a...);
 }
 }  // namespace ych
 
 template <int C, int MB>
 void YC<C, MB>::lapv(const Dev &d, cudaStream_t s) {
-  if (d.prec) ych::go<MB>(ych::c_lapv<float2, C, MB>, d, 1, true, 0, s, d);
-  else ych::go<MB>(ych::c_lapv<double2, C, MB>, d, 1, true, 0, s, d);
+  if (d.prec) ych::go<MB>(ych::c_lapv<float2, C, MB>, d, 1, true, 1, 0, s);
+  else ych::go<MB>(ych::c_lapv<double2, C, MB>, d, 1, true, 1, 0, s);
 }
 template <int C, int MB>
 void YC<C, MB>::assemble(const Dev &d, int rk, cudaStream_t s) {
-  if (d.prec) ych::go<MB>(ych::c_assemble<float2, C, MB, false>, d, 1, false, 0, s, d, rk);
-  else if (d.variant) ych::go<MB>(ych::c_assemble<double2, C, MB, true>, d, 1, false, 0, s, d, rk);
-  else ych::go<MB>(ych::c_assemble<double2, C, MB, false>, d, 1, false, 0, s, d, rk);
+  if (d.prec) ych::go<MB>(ych::c_assemble<float2, C, MB, false>, d, 1, false, 1, 0, s, rk);
+  else if (d.variant) ych::go<MB>(ych::c_assemble<double2, C, MB, true>, d, 1, false, 1, 0, s, rk);
+  else ych::go<MB>(ych::c_assemble<double2, C, MB, false>, d, 1, false, 1, 0, s, rk);
 }
 template <int C, int MB>
 void YC<C, MB>::tder(const Dev &d, bool z, cudaStream_t s) {
-  if (z) {
-    if (d.prec) ych::go<MB>(ych::c_tder<float2, C, MB, false, true>, d, 2, false, 0, s, d);
-    else ych::go<MB>(ych::c_tder<double2, C, MB, false, true>, d, 2, false, 0, s, d);
-  } else if (d.prec) {
-    ych::go<MB>(ych::c_tder<float2, C, MB, false, false>, d, 2, false, 0, s, d);
-  } else if (d.variant) {
-    ych::go<MB>(ych::c_tder<double2, C, MB, true, false>, d, 2, false, 0, s, d);
-  } else {
-    ych::go<MB>(ych::c_tder<double2, C, MB, false, false>, d, 2, false, 0, s, d);
-  }
+  using namespace ych;
+  auto run = [&](auto t) {
+    constexpr int TAB = decltype(t)::value;
+    if (z) {
+      if (d.prec) go<MB>(c_tder<float2, C, MB, false, true, TAB>, d, 2, false, TAB, 0, s);
+      else go<MB>(c_tder<double2, C, MB, false, true, TAB>, d, 2, false, TAB, 0, s);
+    } else if (d.prec) {
+      go<MB>(c_tder<float2, C, MB, false, false, TAB>, d, 2, false, TAB, 0, s);
+    } else if (d.variant) {
+      go<MB>(c_tder<double2, C, MB, true, false, TAB>, d, 2, false, TAB, 0, s);
+    } else {
+      go<MB>(c_tder<double2, C, MB, false, false, TAB>, d, 2, false, TAB, 0, s);
+    }
+  };
+  if (many_waves<MB>(d)) run(std::integral_constant<int, 2>());
+  else run(std::integral_constant<int, 1>());
 }
 template <int C, int MB>
 void YC<C, MB>::sgrad(const Dev &d, cudaStream_t s) {  // mixed: one more block for the exact 00 profiles
-  if (d.prec) ych::go<MB>(ych::c_sgrad<float2, C, MB>, d, 1, false, 1, s, d);
-  else ych::go<MB>(ych::c_sgrad<double2, C, MB>, d, 1, false, 0, s, d);
+  if (d.prec) ych::go<MB>(ych::c_sgrad<float2, C, MB>, d, 1, false, 1, 1, s);
+  else ych::go<MB>(ych::c_sgrad<double2, C, MB>, d, 1, false, 1, 0, s);
 }
 template <int C, int MB>
 void YC<C, MB>::post(const Dev &d, int rk, bool tu, cudaStream_t s) {
-  if (d.prec) {
-    if (tu) ych::go<MB>(ych::c_post<float2, C, MB, true>, d, 2, false, 0, s, d, rk);
-    else ych::go<MB>(ych::c_post<float2, C, MB, false>, d, 2, false, 0, s, d, rk);
-  } else {
-    if (tu) ych::go<MB>(ych::c_post<double2, C, MB, true>, d, 2, false, 0, s, d, rk);
-    else ych::go<MB>(ych::c_post<double2, C, MB, false>, d, 2, false, 0, s, d, rk);
-  }
+  using namespace ych;
+  auto run = [&](auto t) {
+    constexpr int TAB = decltype(t)::value;
+    if (d.prec) {
+      if (tu) go<MB>(c_post<float2, C, MB, true, TAB>, d, 2, false, TAB, 0, s, rk);
+      else go<MB>(c_post<float2, C, MB, false, TAB>, d, 2, false, TAB, 0, s, rk);
+    } else {
+      if (tu) go<MB>(c_post<double2, C, MB, true, TAB>, d, 2, false, TAB, 0, s, rk);
+      else go<MB>(c_post<double2, C, MB, false, TAB>, d, 2, false, TAB, 0, s, rk);
+    }
+  };
+  if (many_waves<MB>(d)) run(std::integral_constant<int, 2>());
+  else run(std::integral_constant<int, 1>());
 }
 template <int C, int MB>
 void YC<C, MB>::psi(const Dev &d, int rk, cudaStream_t s) {
-  if (d.prec) ych::go<MB>(ych::c_psi<float2, C, MB, false>, d, 1, true, 0, s, d, rk);
-  else if (d.variant) ych::go<MB>(ych::c_psi<double2, C, MB, true>, d, 1, true, 0, s, d, rk);
-  else ych::go<MB>(ych::c_psi<double2, C, MB, false>, d, 1, true, 0, s, d, rk);
+  if (d.prec) ych::go<MB>(ych::c_psi<float2, C, MB, false>, d, 1, true, 0, 0, s, rk);
+  else if (d.variant) ych::go<MB>(ych::c_psi<double2, C, MB, true>, d, 1, true, 0, 0, s, rk);
+  else ych::go<MB>(ych::c_psi<double2, C, MB, false>, d, 1, true, 0, 0, s, rk);
 }
 template <int C, int MB>
 void YC<C, MB>::op_y(const Dev &d, int op, const double2 *in, double2 *out, double2 *out2, cudaStream_t s) {
-  ych::go<MB>(ych::c_op<C, MB>, d, 2, true, 0, s, d, op, in, out, out2);
+  ych::go<MB>(ych::c_op<C, MB>, d, 2, true, 2, 0, s, op, in, out, out2);
 }
 template <int C, int MB>
 cudaError_t YC<C, MB>::optin(int limit) {
   using namespace ych;
   const void *fns[] = {(const void *)c_lapv<float2, C, MB>, (const void *)c_lapv<double2, C, MB>,
                        (const void *)c_assemble<float2, C, MB, false>, (const void *)c_assemble<double2, C, MB, true>,
-                       (const void *)c_assemble<double2, C, MB, false>, (const void *)c_tder<float2, C, MB, false, true>,
-                       (const void *)c_tder<double2, C, MB, false, true>, (const void *)c_tder<float2, C, MB, false, false>,
-                       (const void *)c_tder<double2, C, MB, true, false>, (const void *)c_tder<double2, C, MB, false, false>,
+                       (const void *)c_assemble<double2, C, MB, false>, (const void *)c_tder<float2, C, MB, false, true, 1>,
+                       (const void *)c_tder<double2, C, MB, false, true, 1>, (const void *)c_tder<float2, C, MB, false, false, 1>,
+                       (const void *)c_tder<double2, C, MB, true, false, 1>, (const void *)c_tder<double2, C, MB, false, false, 1>,
+                       (const void *)c_tder<float2, C, MB, false, true, 2>, (const void *)c_tder<double2, C, MB, false, true, 2>,
+                       (const void *)c_tder<float2, C, MB, false, false, 2>, (const void *)c_tder<double2, C, MB, true, false, 2>,
+                       (const void *)c_tder<double2, C, MB, false, false, 2>,
                        (const void *)c_sgrad<float2, C, MB>, (const void *)c_sgrad<double2, C, MB>,
-                       (const void *)c_post<float2, C, MB, true>, (const void *)c_post<float2, C, MB, false>,
-                       (const void *)c_post<double2, C, MB, true>, (const void *)c_post<double2, C, MB, false>,
+                       (const void *)c_post<float2, C, MB, true, 1>, (const void *)c_post<float2, C, MB, false, 1>,
+                       (const void *)c_post<double2, C, MB, true, 1>, (const void *)c_post<double2, C, MB, false, 1>,
+                       (const void *)c_post<float2, C, MB, true, 2>, (const void *)c_post<float2, C, MB, false, 2>,
+                       (const void *)c_post<double2, C, MB, true, 2>, (const void *)c_post<double2, C, MB, false, 2>,
                        (const void *)c_psi<float2, C, MB, false>, (const void *)c_psi<double2, C, MB, true>,
                        (const void *)c_psi<double2, C, MB, false>, (const void *)c_op<C, MB>};
   for (const void *fn : fns) {
