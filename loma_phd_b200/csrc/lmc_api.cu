@@ -861,6 +861,7 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
     if (side) {  // beside the RK3 update, which neither reads nor writes what these write
       if (!fork()) return LMC_ECUDA;
       run(6, s2, [&] { lmc::launch_post1_00(d, rk, do_cfl, 1, s2); });
+      run(8, s2, [&] { lmc::launch_psi_tail(d, rk, cfl_step, s2); });
       if (d.tpm) run(6, s2, [&] { lmc::launch_tupd(d, rk, s2); });   // T += Delta T
       if (d.scalar) run(5, s2, [&] { lmc::launch_zupd(d, s2); });    // Z += Delta Z
       run(8, s2, [&] { lmc::launch_psi(d, rk, s2); });
@@ -874,8 +875,8 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
       run(5, s, [&] { lmc::launch_zfwd(d, s, 1); });
       run(7, s, [&] { lmc::launch_post(d, rk, s); });
       run(8, s, [&] { lmc::launch_psi(d, rk, s); });
+      run(8, s, [&] { lmc::launch_psi_tail(d, rk, cfl_step, s); });
     }
-    run(8, s, [&] { lmc::launch_psi_tail(d, rk, cfl_step, s); });
     if (d.prec) {
       d.mean_ok = 1;
       h->mo_flip = 1 - h->mo_flip;

@@ -110,7 +110,8 @@ struct Dev {
   int visc;
   double sigma;
   double *rhst;
-  // device scalars: [0] Deltat, [1] dtr, [2] time, [3] rhobot, [4] rhotop
+  // device scalars: [0] Deltat, [1] dtr, [2] time, [3] rhobot, [4] rhotop,
+  // [5], [6] wall values of Z, [7] Deltat kept for post_dt
   double *scal_d;
   unsigned long long *cflmax;  // [4] max|u|, max|v|/hy, max|w|, max cflT (ordered bits)
   double *rhom;                // [my] plane sums of 1/T
@@ -226,6 +227,12 @@ template <typename CT>
 __device__ __forceinline__ CT *wzb(const Dev &d, int i) {
   if constexpr (sizeof(CT) == sizeof(double2)) return d.zb[i];
   else return d.zbf[i];
+}
+// Deltat for the RK3 update of Omega_y and phi, which may run beside the end
+// of the step (k_psi_00): the copy kept since substep 1 when that sets the
+// next Deltat
+__device__ __forceinline__ double post_dt(const Dev &d, int rk) {
+  return d.scal_d[rk == 2 && !d.variant ? 7 : 0];
 }
 template <typename CT>
 __device__ __forceinline__ const CT *wtwx(const Dev &d) {

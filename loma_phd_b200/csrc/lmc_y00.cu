@@ -172,10 +172,11 @@ __global__ void __launch_bounds__(32, 1) k_psi_00(Dev d, int rk, int cfl_step) {
   if (L.lane == 0) {
     d.diag[5] = trapz;
     d.diag[7] = mu; d.diag[8] = mv; d.diag[9] = mw;
+    if (rk == 1) d.scal_d[7] = dt;
     if (rk == 2) {  // end of the time step: cross.f:1196-1204
       d.diag[0] = d.scal_d[2];
       d.diag[1] = dt;
-      d.scal_d[2] += dt;
+      d.scal_d[2] += dt;  // the RK3 update beside this kernel reads scal_d[7]
       if (cfl_step) d.scal_d[0] = d.scal_d[1];
       d.diag[12] = d.scal_d[0];
     }

@@ -52,13 +52,13 @@ struct Th {
   bool act;                 // the mode exists
   double kx, kz, k2;
   size_t ld;
-  __device__ __forceinline__ Th(const Dev &d) {
+  __device__ __forceinline__ Th(const Dev &d, int blk) {
     ml = threadIdx.x % MB;
     c = threadIdx.x / MB;
     nc = blockDim.x / MB;
     j0 = c * C;
     n = min(C, d.my - j0);
-    const int mm = blockIdx.x * MB + ml;
+    const int mm = blk * MB + ml;
     act = mm < d.nmode;
     m = act ? mm : d.nmode - 1;
     ld = (size_t)d.nmode;
@@ -556,7 +556,7 @@ __device__ __forceinline__ double2 mo00(const Dev &d, int o, int j) {
 
 #define LMC_YC_PROLOGUE(F, POISSON, TAB)               \
   extern __shared__ __align__(16) unsigned char raw[]; \
-  const Th<C, MB> T(d);                                \
+  const Th<C, MB> T(d, blockIdx.x);                    \
   Sm<MB> S;                                            \
   S.template init<TAB>(d, T.nc, F, POISSON, raw);
 
@@ -747,11 +747,16 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_tder(Dev d) {
 // The mixed forms launch one block more: its modes 0, 1, 2 are the exact
 // 00 profiles of rho u, rho v, rho w (mi rows 0..2), differentiated into mi
 // rows 9, 8, 10; the FP32 buffers' 00 coefficients are not read (the
-// transforms drop them).
+// transforms drop them).  parts = 3: a block forms one of the derivatives
+// (sgrad_parts).
 // ----------------------------------------------------------------------
 template <typename CT, int C, int MB>
-__global__ void __launch_bounds__(YC_TMAX, 1) c_sgrad(Dev d) {
-  LMC_YC_PROLOGUE(1, false, 1)
+__global__ void __launch_bounds__(YC_TMAX, 1) c_sgrad(Dev d, int parts) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  const int part = parts == 3 ? (int)blockIdx.x % 3 : -1;
+  const Th<C, MB> T(d, parts == 3 ? blockIdx.x / 3 : blockIdx.x);
+  Sm<MB> S;
+  S.template init<1>(d, T.nc, 1, false, raw);
   double2 x[1][C];
   if constexpr (mixed<CT>()) {
     if (blockIdx.x == gridDim.x - 1) {
@@ -775,31 +780,37 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_sgrad(Dev d) {
     }
   }
   const CT *RU = wsb<CT>(d, SB_RU), *RV = wsb<CT>(d, SB_RV), *RW = wsb<CT>(d, SB_RW);
-  auto deriv = [&](const CT *f, bool first) {
+  S.tables1();
+  auto deriv = [&](const CT *f) {
     double2 u[C + 6];
     rows_h(d, T, f, u);
-    if (first) S.tables1();
     d1_fwd(d, T, S, 0, u, x[0]);
     d1_rest(d, T, S, x);
   };
-  deriv(RV, true);
-  store(T, wsb<CT>(d, SB_GYY), x[0]);
-  deriv(RU, false);
   double2 v[C];
-  rows(T, RV, v);
+  if (part <= 0) {
+    deriv(RV);
+    store(T, wsb<CT>(d, SB_GYY), x[0]);
+    rows(T, RU, v);
+    rows(T, RW, x[0]);
 #pragma unroll
-  for (int t = 0; t < C; t++) x[0][t] = cadd(x[0][t], cik(T.kx, v[t]));
-  store(T, wsb<CT>(d, SB_G12), x[0]);
-  deriv(RW, false);
-  rows(T, RV, v);
+    for (int t = 0; t < C; t++) x[0][t] = cadd(cik(T.kz, v[t]), cik(T.kx, x[0][t]));
+    store(T, wsb<CT>(d, SB_G13), x[0]);
+  }
+  if (part == -1 || part == 1) {
+    deriv(RU);
+    rows(T, RV, v);
 #pragma unroll
-  for (int t = 0; t < C; t++) x[0][t] = cadd(x[0][t], cik(T.kz, v[t]));
-  store(T, wsb<CT>(d, SB_G23), x[0]);
-  rows(T, RU, v);
-  rows(T, RW, x[0]);
+    for (int t = 0; t < C; t++) x[0][t] = cadd(x[0][t], cik(T.kx, v[t]));
+    store(T, wsb<CT>(d, SB_G12), x[0]);
+  }
+  if (part == -1 || part == 2) {
+    deriv(RW);
+    rows(T, RV, v);
 #pragma unroll
-  for (int t = 0; t < C; t++) x[0][t] = cadd(cik(T.kz, v[t]), cik(T.kx, x[0][t]));
-  store(T, wsb<CT>(d, SB_G13), x[0]);
+    for (int t = 0; t < C; t++) x[0][t] = cadd(x[0][t], cik(T.kz, v[t]));
+    store(T, wsb<CT>(d, SB_G23), x[0]);
+  }
 }
 
 // ----------------------------------------------------------------------
@@ -816,12 +827,18 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_sgrad(Dev d) {
 //              - lap((curl omega)_y)/Re,   q = i kx uv + i kz vw
 // (products rho u_i u_j): four first derivatives instead of six, and no
 // N_i or curl goes through memory.  TU: T += Delta T as well (cross.f:
-// 619-627); grids with many modes leave that to c_tupd on the second stream.
+// 619-627); grids with many modes leave that to k_tupd on the second stream.
+// halves = 2: even blocks take RHS(phi), odd ones RHS(Omega_y) (post_halves);
+// neither reads what the other writes.
 // ----------------------------------------------------------------------
 template <typename CT, int C, int MB, bool TU, int TAB>
-__global__ void __launch_bounds__(YC_TMAX, 1) c_post(Dev d, int rk) {
-  LMC_YC_PROLOGUE(2, false, TAB)
-  const double kx = T.kx, kz = T.kz, k2 = T.k2, dtg = d.scal_d[0] * d.gama[rk];
+__global__ void __launch_bounds__(YC_TMAX, 1) c_post(Dev d, int rk, int halves) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  const int half = halves == 2 ? (int)blockIdx.x & 1 : -1;
+  const Th<C, MB> T(d, halves == 2 ? blockIdx.x >> 1 : blockIdx.x);
+  Sm<MB> S;
+  S.template init<TAB>(d, T.nc, 2, false, raw);
+  const double kx = T.kx, kz = T.kz, k2 = T.k2, dtg = post_dt(d, rk) * d.gama[rk];
   const CT *U = wsb<CT>(d, OU), *V = wsb<CT>(d, OV), *W = wsb<CT>(d, OW);
   const CT *UU = wsb<CT>(d, ORUU), *VV = wsb<CT>(d, ORVV), *WW = wsb<CT>(d, ORWW);
   const CT *UV = wsb<CT>(d, ORUV), *UW = wsb<CT>(d, ORUW), *VW = wsb<CT>(d, ORVW);
@@ -838,7 +855,7 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_post(Dev d, int rk) {
     }
   };
   const size_t o = (size_t)T.j0 * T.ld + T.m;
-  {  // RHS(phi)
+  if (half != 1) {  // RHS(phi)
     double2 x[2][C];
     {
       double2 u[C + 6];
@@ -887,12 +904,17 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_post(Dev d, int rk) {
 #pragma unroll
     for (int t = 0; t < C; t++) x[1][t] = fma2(x[1][t], dtg, a[0][t]);  // cross.f:978
     store(T, d.phi, x[1]);
+    if (half == 0) return;
   }
   {  // RHS(Omega_y)
     double2 a[1][C], b[C];
     {
       double2 u[C + 6];
       comb(kz, UV, -kx, VW, u);
+      if (half == 1) {
+        S.tables1();
+        S.tables2();
+      }
       d1_fwd(d, T, S, 0, u, a[0]);
       comb(kz, U, -kx, W, u);
       d2_fwd(d, T, S, 1, k2, u, b);
@@ -1047,7 +1069,22 @@ template <int MB>
 bool many_waves(const Dev &d) {
   return (d.nmode + MB - 1) / MB > 4 * 148;
 }
-// One block per MB modes (and `extra`), shared memory for F pencils and for
+// Blocks of nt threads that the registers of the device hold (128 each).
+inline int resident(int nt) { return std::max(64 / ((nt + 31) / 32 * 4), 1) * 148; }
+// c_post as two blocks per MB modes, one for each right-hand side: shorter
+// chains where twice the blocks still run at once (24 x 25 x 24: 0.173 ms per
+// step against 0.205; 512 x 257 2-D 0.618 against 0.627), and shorter last
+// waves where they come in waves anyway (12,192 x 193: 4.97 against 5.24;
+// 8,128 x 129 2.40 against 2.45; 6,096 x 129 with the scalar and mu 2.53
+// against 2.65).  In between the second wave costs more (2,016 x 129 with
+// both: 0.93 against 0.88).
+inline int post_halves(int g, int nt) { return 2 * g <= resident(nt) || g > resident(nt) ? 2 : 1; }
+// c_sgrad as three, one for each derivative, where they all run at once
+// (1,128 modes x 97: 0.525 ms per step against 0.560; 4,560 x 97, where they
+// do not: 1.472 against 1.461).
+inline int sgrad_parts(int g, int nt) { return 3 * g <= resident(nt) ? 3 : 1; }
+
+// `parts` blocks per MB modes (and `extra` blocks), shared memory for F pencils and for
 // the tables of d/dy (tabs 1) and of d2/dy2 (tabs 2), which every block reads
 // several times: from global memory they come out of the L2 with each pass,
 // as the pencils' rows push them out of the L1 (c_post, 12,192 x 193: 16 of
@@ -1057,13 +1094,12 @@ bool many_waves(const Dev &d) {
 // 64 x 129 x 64 with the scalar and mu 0.93 after 1.00; 96 x 129 x 96, float2
 // buffers, 1.29 after 1.33; 192 x 193 x 128 5.29 after 5.60.
 template <int MB, typename K, typename... A>
-void go(K k, const Dev &d, int F, bool poisson, int tabs, int extra, cudaStream_t s, A... a) {
-  const int g = (d.nmode + MB - 1) / MB + extra, nt = d.ync * MB;
+void go(K k, const Dev &d, int F, bool poisson, int tabs, int parts, int extra, cudaStream_t s, A... a) {
+  const int g = (d.nmode + MB - 1) / MB * parts + extra, nt = d.ync * MB;
   const size_t base = Sm<MB>::bytes(d.ync, F, poisson);
   const size_t tab = sizeof(double) * (tabs == 2 ? d.ct.n1 + d.ct.n2 : tabs == 1 ? d.ct.n1 : 0);
   const size_t sm = 228 * 1024, res = 1024;                // shared memory of an SM, and what each block reserves of it
-  size_t per = 64 / ((nt + 31) / 32 * 4);  // blocks by registers (128 each)
-  per = std::min(std::max<size_t>(per, 1), std::min<size_t>(sm / (base + res), (g + 147) / 148));
+  const size_t per = std::min<size_t>(resident(nt) / 148, std::min<size_t>(sm / (base + res), (g + 147) / 148));
   Dev e = d;
   e.ct.sm = tab > 0 && base + tab <= (size_t)d.smem_limit && per * (base + tab + res) <= sm;
   k<<<g, nt, base + (e.ct.sm ? tab : 0), s>>>(e, a...);
@@ -1072,14 +1108,14 @@ void go(K k, const Dev &d, int F, bool poisson, int tabs, int extra, cudaStream_
 
 template <int C, int MB>
 void YC<C, MB>::lapv(const Dev &d, cudaStream_t s) {
-  if (d.prec) ych::go<MB>(ych::c_lapv<float2, C, MB>, d, 1, true, 1, 0, s);
-  else ych::go<MB>(ych::c_lapv<double2, C, MB>, d, 1, true, 1, 0, s);
+  if (d.prec) ych::go<MB>(ych::c_lapv<float2, C, MB>, d, 1, true, 1, 1, 0, s);
+  else ych::go<MB>(ych::c_lapv<double2, C, MB>, d, 1, true, 1, 1, 0, s);
 }
 template <int C, int MB>
 void YC<C, MB>::assemble(const Dev &d, int rk, cudaStream_t s) {
-  if (d.prec) ych::go<MB>(ych::c_assemble<float2, C, MB, false>, d, 1, false, 1, 0, s, rk);
-  else if (d.variant) ych::go<MB>(ych::c_assemble<double2, C, MB, true>, d, 1, false, 1, 0, s, rk);
-  else ych::go<MB>(ych::c_assemble<double2, C, MB, false>, d, 1, false, 1, 0, s, rk);
+  if (d.prec) ych::go<MB>(ych::c_assemble<float2, C, MB, false>, d, 1, false, 1, 1, 0, s, rk);
+  else if (d.variant) ych::go<MB>(ych::c_assemble<double2, C, MB, true>, d, 1, false, 1, 1, 0, s, rk);
+  else ych::go<MB>(ych::c_assemble<double2, C, MB, false>, d, 1, false, 1, 1, 0, s, rk);
 }
 template <int C, int MB>
 void YC<C, MB>::tder(const Dev &d, bool z, cudaStream_t s) {
@@ -1087,14 +1123,14 @@ void YC<C, MB>::tder(const Dev &d, bool z, cudaStream_t s) {
   auto run = [&](auto t) {
     constexpr int TAB = decltype(t)::value;
     if (z) {
-      if (d.prec) go<MB>(c_tder<float2, C, MB, false, true, TAB>, d, 2, false, TAB, 0, s);
-      else go<MB>(c_tder<double2, C, MB, false, true, TAB>, d, 2, false, TAB, 0, s);
+      if (d.prec) go<MB>(c_tder<float2, C, MB, false, true, TAB>, d, 2, false, TAB, 1, 0, s);
+      else go<MB>(c_tder<double2, C, MB, false, true, TAB>, d, 2, false, TAB, 1, 0, s);
     } else if (d.prec) {
-      go<MB>(c_tder<float2, C, MB, false, false, TAB>, d, 2, false, TAB, 0, s);
+      go<MB>(c_tder<float2, C, MB, false, false, TAB>, d, 2, false, TAB, 1, 0, s);
     } else if (d.variant) {
-      go<MB>(c_tder<double2, C, MB, true, false, TAB>, d, 2, false, TAB, 0, s);
+      go<MB>(c_tder<double2, C, MB, true, false, TAB>, d, 2, false, TAB, 1, 0, s);
     } else {
-      go<MB>(c_tder<double2, C, MB, false, false, TAB>, d, 2, false, TAB, 0, s);
+      go<MB>(c_tder<double2, C, MB, false, false, TAB>, d, 2, false, TAB, 1, 0, s);
     }
   };
   if (many_waves<MB>(d)) run(std::integral_constant<int, 2>());
@@ -1102,20 +1138,22 @@ void YC<C, MB>::tder(const Dev &d, bool z, cudaStream_t s) {
 }
 template <int C, int MB>
 void YC<C, MB>::sgrad(const Dev &d, cudaStream_t s) {  // mixed: one more block for the exact 00 profiles
-  if (d.prec) ych::go<MB>(ych::c_sgrad<float2, C, MB>, d, 1, false, 1, 1, s);
-  else ych::go<MB>(ych::c_sgrad<double2, C, MB>, d, 1, false, 1, 0, s);
+  const int parts = ych::sgrad_parts((d.nmode + MB - 1) / MB, d.ync * MB);
+  if (d.prec) ych::go<MB>(ych::c_sgrad<float2, C, MB>, d, 1, false, 1, parts, 1, s, parts);
+  else ych::go<MB>(ych::c_sgrad<double2, C, MB>, d, 1, false, 1, parts, 0, s, parts);
 }
 template <int C, int MB>
 void YC<C, MB>::post(const Dev &d, int rk, bool tu, cudaStream_t s) {
   using namespace ych;
+  const int g = (d.nmode + MB - 1) / MB, halves = post_halves(g, d.ync * MB);
   auto run = [&](auto t) {
     constexpr int TAB = decltype(t)::value;
     if (d.prec) {
-      if (tu) go<MB>(c_post<float2, C, MB, true, TAB>, d, 2, false, TAB, 0, s, rk);
-      else go<MB>(c_post<float2, C, MB, false, TAB>, d, 2, false, TAB, 0, s, rk);
+      if (tu) go<MB>(c_post<float2, C, MB, true, TAB>, d, 2, false, TAB, halves, 0, s, rk, halves);
+      else go<MB>(c_post<float2, C, MB, false, TAB>, d, 2, false, TAB, halves, 0, s, rk, halves);
     } else {
-      if (tu) go<MB>(c_post<double2, C, MB, true, TAB>, d, 2, false, TAB, 0, s, rk);
-      else go<MB>(c_post<double2, C, MB, false, TAB>, d, 2, false, TAB, 0, s, rk);
+      if (tu) go<MB>(c_post<double2, C, MB, true, TAB>, d, 2, false, TAB, halves, 0, s, rk, halves);
+      else go<MB>(c_post<double2, C, MB, false, TAB>, d, 2, false, TAB, halves, 0, s, rk, halves);
     }
   };
   if (many_waves<MB>(d)) run(std::integral_constant<int, 2>());
@@ -1123,13 +1161,13 @@ void YC<C, MB>::post(const Dev &d, int rk, bool tu, cudaStream_t s) {
 }
 template <int C, int MB>
 void YC<C, MB>::psi(const Dev &d, int rk, cudaStream_t s) {
-  if (d.prec) ych::go<MB>(ych::c_psi<float2, C, MB, false>, d, 1, true, 0, 0, s, rk);
-  else if (d.variant) ych::go<MB>(ych::c_psi<double2, C, MB, true>, d, 1, true, 0, 0, s, rk);
-  else ych::go<MB>(ych::c_psi<double2, C, MB, false>, d, 1, true, 0, 0, s, rk);
+  if (d.prec) ych::go<MB>(ych::c_psi<float2, C, MB, false>, d, 1, true, 0, 1, 0, s, rk);
+  else if (d.variant) ych::go<MB>(ych::c_psi<double2, C, MB, true>, d, 1, true, 0, 1, 0, s, rk);
+  else ych::go<MB>(ych::c_psi<double2, C, MB, false>, d, 1, true, 0, 1, 0, s, rk);
 }
 template <int C, int MB>
 void YC<C, MB>::op_y(const Dev &d, int op, const double2 *in, double2 *out, double2 *out2, cudaStream_t s) {
-  ych::go<MB>(ych::c_op<C, MB>, d, 2, true, 2, 0, s, op, in, out, out2);
+  ych::go<MB>(ych::c_op<C, MB>, d, 2, true, 2, 1, 0, s, op, in, out, out2);
 }
 template <int C, int MB>
 cudaError_t YC<C, MB>::optin(int limit) {

@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(YS_TB) t_sgrad(Dev d) {
 // ----------------------------------------------------------------------
 template <typename CT>
 __global__ void __launch_bounds__(YS_TB) t_post(Dev d, int rk) {
-  const double dtg = d.scal_d[0] * d.gama[rk];
+  const double dtg = post_dt(d, rk) * d.gama[rk];
   LMC_SWEEP_MODE
   {
     const double kx = M.kx, kz = M.kz, k2 = M.k2;

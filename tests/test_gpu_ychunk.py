@@ -6,7 +6,7 @@ many modes with a last block that is not full, against the FP64 oracle.
 Bars, those of the operator and step parity tests: operators <= 1e-12
 (relative L2; above the 129 points those tests go to, times (ny/129)^2, as the
 condition of the second-order operators grows), one RK3 step <= 1e-10 per
-field (FP64) and <= 1e-6 (mixed).
+field (FP64) and <= 1e-6 (mixed; 3e-6 with the variable viscosity).
 """
 import numpy as np
 import pytest
@@ -74,7 +74,8 @@ def test_operators(gpu, monkeypatch, nx, nz, ny, path):
 
 
 @pytest.mark.parametrize("prec,tol", [(0, 1e-10), (1, 1e-6)])
-@pytest.mark.parametrize("nx,nz,ny,path", [GRIDS[0], GRIDS[3], GRIDS[6], GRIDS[7], (24, 32, 300, "warp"), GRIDS[8], GRIDS[9]])
+@pytest.mark.parametrize("nx,nz,ny,path", [GRIDS[0], GRIDS[3], GRIDS[6], GRIDS[7], (24, 32, 300, "warp"), (64, 96, 129, "warp"),
+                                          GRIDS[-2], GRIDS[-1]])
 def test_one_step(gpu, monkeypatch, nx, nz, ny, path, prec, tol):
     _path(monkeypatch, path)
     p, y, st = case(nx=nx, nz=nz, ny=ny, precision=prec)
@@ -87,4 +88,24 @@ def test_one_step(gpu, monkeypatch, nx, nz, ny, path, prec, tol):
     o.step(1)
     so = o.get_state()
     for k in FIELDS + ("u00", "v00"):
+        assert rel_l2(sg[k], so[k]) < tol, (k, rel_l2(sg[k], so[k]))
+
+
+@pytest.mark.parametrize("prec,tol", [(0, 1e-10), (1, 3e-6)])
+@pytest.mark.parametrize("nx,nz,ny", [(16, 16, 31), (64, 96, 129)])
+def test_one_step_visc(gpu, monkeypatch, nx, nz, ny, prec, tol):
+    """The strain-rate inputs from three blocks per group of modes, and from one."""
+    _path(monkeypatch, "warp")
+    kw = dict(nx=nx, nz=nz, ny=ny, visc=1, sigma=0.7)
+    p, y, st = case(precision=prec, **kw)
+    g = Lomacte(p, y)
+    g.load_state(st)
+    g.step(1)
+    sg = g.get_state()
+    g.close()
+    o = oracle_for(case(**kw)[0], y, st)
+    o.set_viscosity(0.7)
+    o.step(1)
+    so = o.get_state()
+    for k in FIELDS + ("u00", "w00"):
         assert rel_l2(sg[k], so[k]) < tol, (k, rel_l2(sg[k], so[k]))
