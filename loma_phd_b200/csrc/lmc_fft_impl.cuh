@@ -71,17 +71,19 @@ struct XGeo {
 // are touched in runs of KB values: 64 bytes from 576 points up (FP64, 1152
 // points, 768 x 33: k_zfwd 3.6 ms per step against 6.4 with 32 bytes; FP32
 // 3.9 against 4.3), 128 at 384 and 288 (256 x 257: FP64 2.9 against 3.7, FP32
-// 1.5 against 1.8), where the lines are short enough to fit.
+// 1.5 against 1.8), where the lines are short enough to fit; KiB at the three
+// points of a 2-D grid, whose blocks are too small to be worth their launch
+// otherwise (512 x 257: k_zfwd 10 us per launch after 50, k_zinv 6 after 20).
 template <int R1, int R2, int R3, typename CT>
 struct ZGeo {
   using F = Fft<R1, R2, R3, CT>;
   static constexpr int N = R1 * R2 * R3, W = sizeof(CT) == sizeof(float2) ? 2 : 1;
-  static constexpr int KB = W * (N == 384 || N == 288 ? 8 : N >= 144 ? 4 : 8);
+  static constexpr int KB = W * (N == 384 || N == 288 ? 8 : N >= 144 ? 4 : N == 3 ? 64 : 8);
   static constexpr int ZI = W * (N == 1152 ? 192 : N == 576 ? 96 : N == 288 ? 96 : N >= 384 ? 128 : 64);
   static constexpr int ZF = W * (N == 1152 ? (W == 2 ? 144 : 192) : N == 576 ? 144 : N == 288 ? 96 : N >= 384 ? 128 : 64);
   static constexpr int MI = (W == 2 ? 768 : 512) / ZI, MF = (W == 2 ? 768 : 512) / ZF;
   static constexpr int UN = 128 / (int)sizeof(CT), OD = F::RUN + 1, ST = KB >= UN ? 1 : UN / KB;
-  static constexpr int LD = F::LD + ((ST * OD) % UN + UN - F::LD % UN) % UN;
+  static constexpr int LD = N == 3 ? 3 : F::LD + ((ST * OD) % UN + UN - F::LD % UN) % UN;
 };
 
 __host__ __device__ constexpr size_t round16(size_t b) { return (b + 15) / 16 * 16; }
