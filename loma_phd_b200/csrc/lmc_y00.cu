@@ -3,8 +3,8 @@
 //
 // One pencil per warp: its my points are split over the lanes in chunks and
 // the banded solves join the chunks by shuffles (lmc_device.cuh), so each of
-// these one-block kernels is a short chain of latencies.  The five banded
-// operators that the 00 right-hand sides need run on five warps at once.
+// these one-block kernels is a short chain of latencies.  The six banded
+// operators that the 00 modes need run on six warps at once.
 #include <cuda_runtime.h>
 
 #include "lmc_kernels.cuh"
@@ -64,10 +64,14 @@ __device__ __forceinline__ void load00(const Dev &d, int o, const Lane &L, doubl
 }
 
 // dw, dm, masst, the 00 RHS of rho u00 / rho w00, H00 and the CFL Deltat:
-// cross.f:686-722, 1416-1429, 1778-1826.  Warps 0 and 1: d2/dy2 of u00 and
-// w00; 2 and 3: d/dy of rho uv and rho vw; 4: the thicknesses and the mass.
+// cross.f:686-722, 1416-1429, 1778-1826, and the integral of d(rho)/dt00 for
+// rho v00 (inty8).  Warps 0 and 1: d2/dy2 of u00 and w00; 2 and 3: d/dy of
+// rho uv and rho vw; 4: the thicknesses and the mass; 5: inty8, which had its
+// turn in k_psi_00 before, so that this kernel, k_psi_00 and c_psi in a row
+// took longer than the RK3 update beside them (512 x 257 2-D: 0.40 ms per
+// step after 0.42; 192 x 193 x 128 4.94 after 4.97).
 template <int C, typename CT>
-__global__ void __launch_bounds__(160, 1) k_post1_00(Dev d, int rk, int do_cfl, int do_diag) {
+__global__ void __launch_bounds__(192, 1) k_post1_00(Dev d, int rk, int do_cfl, int do_diag) {
   extern __shared__ double R[];  // [4][my]
   const Lane L = make_lane<C>(d.lpm, d.base, d.extra);
   const int w = threadIdx.x >> 5, my = d.my;
@@ -79,6 +83,20 @@ __global__ void __launch_bounds__(160, 1) k_post1_00(Dev d, int rk, int do_cfl, 
 #pragma unroll
     for (int t = 0; t < C; t++)
       if (t < L.n) R[w * my + L.s + t] = a[t].x;
+  } else if (w == 5) {
+    if (!d.variant) {  // inty8 (laps.f:484-575): rf0v(y) = int d(rho)/dt00 dy with rf0v(1) = 0
+      load00<C, CT>(d, ODRHO, L, a);
+#pragma unroll
+      for (int t = 0; t < C; t++) a[t] = make_double2((t < L.n) ? a[t].x / tab(d.fmap, 1, t, 0, L.lane) : 0.0, 0.0);
+      matvec_ip<C, 3>(d.dt11, L, a);
+      lsolve_c<C, 3>(a, d.i8L, d.k8L, L);
+      usolve_c<C, 3>(a, d.i8U, d.k8U, L);
+      const double v0 = bcast_row(a, L, 0).x, vn = bcast_row(a, L, my - 1).x;
+#pragma unroll
+      for (int t = 0; t < C; t++)
+        if (t < L.n) d.rf0v[L.s + t] = a[t].x - v0;
+      if (L.lane == 0) d.diag[5] = -(vn - v0);  // trapz, cross.f:1046
+    }
   } else {
     if (rk == 2 && do_diag) {  // vorticity thickness, cross.f:692-699
       load00<C, CT>(d, OU, L, a);
@@ -129,48 +147,27 @@ __global__ void __launch_bounds__(160, 1) k_post1_00(Dev d, int rk, int do_cfl, 
   }
 }
 
-// rho u00 / rho w00 RK3 update, masses, inty8 of d(rho)/dt00 for rho v00 with
-// the acoustic wall correction, end-of-step time and Deltat: cross.f:
-// 1006-1074, 1196-1204.
-template <int C, typename CT>
+// rho u00 / rho w00 RK3 update, masses, rho v00 with the acoustic wall
+// correction, end-of-step time and Deltat: cross.f:1006-1074, 1196-1204.  One
+// warp, its lanes along y.
 __global__ void __launch_bounds__(32, 1) k_psi_00(Dev d, int rk, int cfl_step) {
-  const Lane L = make_lane<C>(d.lpm, d.base, d.extra);
-  double2 a[C];
-  load00<C, CT>(d, ODRHO, L, a);
   const double dt = d.scal_d[0], dtg = dt * d.gama[rk];
+  const double corr = d.diag[5] / (1.0 + sqrt(d.scal_d[4] / d.scal_d[3]));  // cross.f:1064-1065
   double mu = 0.0, mv = 0.0, mw = 0.0;
-#pragma unroll
-  for (int t = 0; t < C; t++)
-    if (t < L.n) {
-      const int j = L.s + t;
-      if (j >= 1 && j <= d.my - 2) {  // cross.f:1008-1011
-        d.u00[j] += dtg * d.rf0u[j];
-        d.w00[j] += dtg * d.rf0w[j];
-      }
-      const double h = d.hy[j];  // cross.f:1016-1020
-      mu += d.u00[j] * h;
-      mv += d.v00[j] * h;
-      mw += d.w00[j] * h;
-    }
+#pragma unroll 4
+  for (int j = threadIdx.x; j < d.my; j += 32) {
+    const bool in = j >= 1 && j <= d.my - 2;  // cross.f:1008-1011
+    const double h = d.hy[j], ru = d.rf0u[j], rw = d.rf0w[j];
+    const double u = in ? d.u00[j] + dtg * ru : d.u00[j], w = in ? d.w00[j] + dtg * rw : d.w00[j];
+    mu += u * h;  // cross.f:1016-1020
+    mv += d.v00[j] * h;
+    mw += w * h;
+    d.u00[j] = u;
+    d.w00[j] = w;
+    d.v00[j] = d.rf0v[j] + corr;
+  }
   mu = warp_sum(mu); mv = warp_sum(mv); mw = warp_sum(mw);
-  // inty8 (laps.f:484-575): rf0v(y) = int d(rho)/dt00 dy with rf0v(1) = 0
-#pragma unroll
-  for (int t = 0; t < C; t++) a[t] = make_double2((t < L.n) ? a[t].x / tab(d.fmap, 1, t, 0, L.lane) : 0.0, 0.0);
-  matvec_ip<C, 3>(d.dt11, L, a);
-  lsolve_c<C, 3>(a, d.i8L, d.k8L, L);
-  usolve_c<C, 3>(a, d.i8U, d.k8U, L);
-  const double v0 = bcast_row(a, L, 0).x, vn = bcast_row(a, L, d.my - 1).x;
-  const double trapz = -(vn - v0);                                       // cross.f:1046
-  const double corr = trapz / (1.0 + sqrt(d.scal_d[4] / d.scal_d[3]));  // cross.f:1064-1065
-#pragma unroll
-  for (int t = 0; t < C; t++)
-    if (t < L.n) {
-      const double r = a[t].x - v0;
-      d.rf0v[L.s + t] = r;
-      d.v00[L.s + t] = r + corr;
-    }
-  if (L.lane == 0) {
-    d.diag[5] = trapz;
+  if (threadIdx.x == 0) {
     d.diag[7] = mu; d.diag[8] = mv; d.diag[9] = mw;
     if (rk == 1) d.scal_d[7] = dt;
     if (rk == 2) {  // end of the time step: cross.f:1196-1204
@@ -185,13 +182,8 @@ __global__ void __launch_bounds__(32, 1) k_psi_00(Dev d, int rk, int cfl_step) {
 
 template <int C, typename CT>
 void post1_00(const Dev &d, int rk, int do_cfl, int do_diag, cudaStream_t s) {
-  k_post1_00<C, CT><<<1, 160, (size_t)4 * d.my * sizeof(double), s>>>(d, rk, do_cfl, do_diag);
+  k_post1_00<C, CT><<<1, 192, (size_t)4 * d.my * sizeof(double), s>>>(d, rk, do_cfl, do_diag);
 }
-template <int C, typename CT>
-void psi_00(const Dev &d, int rk, int cfl_step, cudaStream_t s) {
-  k_psi_00<C, CT><<<1, 32, 0, s>>>(d, rk, cfl_step);
-}
-
 }  // namespace
 
 // d.C: points per lane (the chunk sizes of pick_chunks)
@@ -212,10 +204,6 @@ void launch_post1_00(const Dev &d, int rk, int do_cfl, int do_diag, cudaStream_t
   LMC_Y00(CALL)
 #undef CALL
 }
-void launch_psi_00(const Dev &d, int rk, int cfl_step, cudaStream_t s) {
-#define CALL(C, CT) psi_00<C, CT>(d, rk, cfl_step, s)
-  LMC_Y00(CALL)
-#undef CALL
-}
+void launch_psi_00(const Dev &d, int rk, int cfl_step, cudaStream_t s) { k_psi_00<<<1, 32, 0, s>>>(d, rk, cfl_step); }
 
 }  // namespace lmc
