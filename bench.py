@@ -67,7 +67,8 @@ PR = float(np.float32(0.7))  # Pr = Sc = 0.7f (main.f:569)
 # R_Omega, R_phi) are FP64 complex (16 B) in both forms; transform work
 # buffers take w bytes per complex value (16 in the FP64 form, 8 in the mixed
 # form).  Compulsory reads + writes of each kernel group (one profile id):
-#   zinv : 6 spectral inputs read (rho u, rho v, rho w, lap T, dT/dy, T), 8 Z written
+#   zinv : 6 spectral inputs read (rho u, rho v, rho w, lap T, dT/dy, T), 8 Z written (dT/dx
+#          and, with vs, d(rho u)/dx among them, which the x stage forms now)
 #   xphys: 8 Z read, 11 Z written, RHS(T) physical accumulator (FP64) read + written
 #   zfwd : 11 Z read, 11 S written
 #   lapv : phi read, m_y and dm_y/dy written (+ 7 doubles/point mode tables read)
@@ -79,11 +80,11 @@ PR = float(np.float32(0.7))  # Pr = Sc = 0.7f (main.f:569)
 #   psi  : drho read, psi written (+ 7 doubles/point mode tables read)
 # The passive scalar (sc) adds to zinv lap Z, dZ/dy, Z read and 4 Z
 # written; to xphys 4 Z read, 1 Z written (the twelfth output) and its
-# physical accumulator; to zfwd the twelfth output; to tder (t_zder) Z read
-# and written, dZ/dy, lap Z written; to zfwd's profile id (t_zupd) Z read
+# physical accumulator; to zfwd the twelfth output; to tder Z read
+# and written, dZ/dy, lap Z written; to zfwd's profile id (k_tupd of Z) Z read
 # and written, Delta Z read.  The variable viscosity (vs) adds to zinv the
 # four strain-rate sums read and 6 Z written; to xphys 6 Z read; to the
-# assemble id (t_sgrad) rho u, rho v, rho w read and the four sums written.
+# assemble id (c_sgrad, t_sgrad) rho u, rho v, rho w read and the four sums written.
 ALGO = {
     "zinv": lambda S, Z, P, w, sc, vs: (6 + 3 * sc + 4 * vs) * S * w + (8 + 4 * sc + 6 * vs) * Z * w,
     "xphys": lambda S, Z, P, w, sc, vs: (19 + 5 * sc + 6 * vs) * Z * w + 2 * (1 + sc) * P * 8,
@@ -102,10 +103,10 @@ ALGO = {
 # kernel's traffic grows in proportion to ny at fixed x/z sizes.  None:
 # not captured for that kernel.
 NCU_TRAFFIC = {
-    # 768^2 x 33 (mgal 1152^2), mu = T^0.7 + scalar: profiles/kernels_transforms_large_768x33x768.md
-    ("large", False, 1, 1): {"xphys": (5.0270e9, 33)},
-    ("large", True, 1, 1): {"xphys": (8.3872e9, 33)},
-    # 256^2 x 65 (mgal 384^2), mu = T^0.7 + scalar: profiles/kernels_xphys_mu07_scalar_256x65x256.md
+    # 768^2 x 17 (mgal 1152^2), mu = T^0.7 + scalar: profiles/kernels_xphys_mu07_scalar_768x17x768.md
+    ("large", False, 1, 1): {"xphys": (2.3682e9, 17)},
+    ("large", True, 1, 1): {"xphys": (4.0450e9, 17)},
+    # 256^2 x 65 (mgal 384^2), mu = T^0.7 + scalar, before dT/dx was formed by the x stage: profiles/kernels_xphys_mu07_scalar_256x65x256.md
     ("medium", False, 1, 1): {"xphys": (1026.2e6, 65)},
     ("medium", True, 1, 1): {"xphys": (1791.0e6, 65)},
 }

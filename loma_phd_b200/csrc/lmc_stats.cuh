@@ -78,7 +78,7 @@ __device__ __forceinline__ double *spec_at(const Dev &d, const Stats &st, int i,
 // ----------------------------------------------------------------------
 // addstats1 (cross.f:1981-2064): spectra of rho u, rho v, rho w, T at the
 // spectra planes, Tp, and the 00 means rum, rvm, rwm, Tm.  T is the state
-// at the start of the substep with its wall values set (k_tder wrote them).
+// at the start of the substep with its wall values set (c_tder or t_tder wrote them).
 // ----------------------------------------------------------------------
 template <typename CT>
 __global__ void __launch_bounds__(SRT) k_srow1(Dev d, Stats st) {
