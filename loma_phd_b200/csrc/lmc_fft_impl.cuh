@@ -303,28 +303,17 @@ __device__ __forceinline__ void x_out(const Dev &d, const CT *sm, int nl, size_t
   });
 }
 
-// The output pairs of the x stage.  The rounding of a packed line is that of
-// the larger of its two fields, white in wavenumber, and the phi equation
-// weights the six products by k^3: they share lines with one another, where
-// their fluctuations are of one size (1e-4 in the middle of a mixing layer
-// with 1 percent of perturbation, where w has 1e-2 and drho 3e-3).  With rho uu
-// beside w and rho vw beside drho phi is further from the FP64 form: after four
-// steps of 768 x 65 x 768 (mu, scalar, FP32 transforms) 6.8e-6 (two-pass
-// transforms), with these pairs 5.7e-6, at the worst mode 1.2e-3 and 7.4e-4
-// of its rms.
-constexpr int pair_list(int a, int b, int c, int d, int e, int f) {
-  return a | b << 4 | c << 8 | d << 12 | e << 16 | f << 20;
-}
-constexpr int X_PAIR_A = pair_list(OU, OW, ORUU, ORVV, ORUV, ODT);
-constexpr int X_PAIR_B = pair_list(OV, ODRHO, ORUW, ORWW, ORVW, ODZ);
-
 // The x stage: per (y, z line), inverse x transforms of the inputs, packed two
 // per complex transform,
 //   (rho u, rho v) (rho w, lap T) (dT/dx, dT/dy) (dT/dz, T)
 //   ZS, the passive scalar: (lap Z, dZ/dx) (dZ/dy, dZ/dz)
 //   VS, the variable viscosity: the strain-rate inputs (vbase) in pairs
 // the FP64 products and the T (and Z) update, and the direct transforms of
-//   (u, v) (w, drho) (rho uu, rho uw) (rho vv, rho ww) (rho uv, rho vw) (DT, DZ)
+//   (u, v) (w, rho uu) (rho vv, rho ww) (rho uv, rho uw) (rho vw, drho) (DT, DZ)
+// (the rounding of a packed FP32 line is that of the larger of its two fields:
+// drho, which vanishes with the density contrast and is all that psi is solved
+// from, shares its line with the smallest product and not with a velocity; at a
+// density ratio of 1.05 psi is 1.1e-7 off beside rho vw and 1.4e-6 beside w),
 // in place: every input row of a tile is read in the first pass, before any
 // output row is written.  dT/dx and d(rho u)/dx are formed from the rows of T
 // and rho u.  VS: T^sigma in the diffusion of T and Z, and the variable part
@@ -543,10 +532,10 @@ __global__ void __launch_bounds__(XGeo<R1, R2, R3, sizeof(CT) == sizeof(float2)>
         vw -= c * (T * g2.y + rv * tz + rw * ty);
       }
       out(0, OU, u, OV, v);
-      out(1, OW, w, ODRHO, drho);
-      out(2, ORUU, uu, ORUW, uw);
-      out(3, ORVV, vv, ORWW, ww);
-      out(4, ORUV, uv, ORVW, vw);
+      out(1, OW, w, ORUU, uu);
+      out(2, ORVV, vv, ORWW, ww);
+      out(3, ORUV, uv, ORUW, uw);
+      out(4, ORVW, vw, ODRHO, drho);
       out(5, ODT, d8, ODZ, dz);                                        // cross.f:1645-1647
       if (do_cfl) {
         mu = fmax(mu, fabs(u));
@@ -594,8 +583,9 @@ __global__ void __launch_bounds__(XGeo<R1, R2, R3, sizeof(CT) == sizeof(float2)>
     F::template fwd_p3<-1>(W, nl * ZB, LD, wtwx<CT>(d));
     F::template fwd_p2<-1>(W, nl * ZB, LD, wtwx<CT>(d));
     x_out<R1, R2, R3, XT, CT, ST>(d, W, nl, gt, nzb, [](int p, int &fa, int &fb) {
-      fa = X_PAIR_A >> 4 * p & 15;
-      fb = p < 5 || ZS ? X_PAIR_B >> 4 * p & 15 : -1;
+      // OU .. ODT in order, two per line; the last line's second is Delta Z
+      fa = 2 * p;
+      fb = p < 5 || ZS ? 2 * p + 1 : -1;
     });
     __syncthreads();
   }
