@@ -116,9 +116,7 @@ int dupload(lmc_handle *h, const T **p, const std::vector<T> &v) {
 // transform's.  C: double2 or float2
 template <typename C>
 std::vector<C> fft_twiddles(int n) {
-  lmc::FftRadix f{n, n, 1, 1};
-  for (const auto &q : lmc::FFT_RADIX)
-    if (q.n == n) f = q;
+  const lmc::FftRadix f = lmc::fft_radix(n, sizeof(C) == sizeof(float2));
   const int M = f.r2 * f.r3;
   std::vector<C> t;
   auto put = [&](long long e, int len) {

@@ -446,11 +446,16 @@ __device__ __forceinline__ int warp_sum12(const double (&a)[12], double (&v)[3])
 // Twiddles exp(-2 pi i e/R) come from a constant table (c_tw), one block
 // per size, filled by the host at initialisation.
 // ---------------------------------------------------------------------
-constexpr int TW_SIZES[] = {4, 6, 8, 12, 16};
+constexpr int TW_SIZES[] = {4, 6, 8, 9, 12, 16, 18, 24, 32, 36, 48};
 __host__ __device__ constexpr int tw_off(int R) {
-  return R == 4 ? 0 : R == 6 ? 4 : R == 8 ? 10 : R == 12 ? 18 : R == 16 ? 30 : -1;
+  int o = 0;
+  for (int q : TW_SIZES) {
+    if (q == R) return o;
+    o += q;
+  }
+  return -1;
 }
-constexpr int TW_TOTAL = 4 + 6 + 8 + 12 + 16;
+constexpr int TW_TOTAL = tw_off(48) + 48;
 
 static __constant__ double2 c_tw[TW_TOTAL];  // one copy per translation unit
 static __constant__ float2 c_twf[TW_TOTAL];  // the same, rounded to FP32
@@ -492,10 +497,21 @@ __device__ __forceinline__ void bfly(CT (&x)[R]) {
   }
 }
 
-template <int R, int SIGN, typename CT>
+// GAP: the middle third of the samples is zero (and not read); the innermost
+// stage, radix 3, takes one sample of each third
+template <int R, int SIGN, bool GAP = false, typename CT>
 __device__ __forceinline__ void rdft(CT (&x)[R]) {
+  static_assert(!GAP || R % 3 == 0, "the gap must be whole samples");
   if constexpr (R == 1) {
     return;
+  } else if constexpr (R == 3 && GAP) {
+    using Re = typename CReal<CT>::R;
+    const Re s3 = (Re)0.86602540378443864676;  // sqrt(3)/2
+    const CT c = x[2], a = cmk<CT>(x[0].x - (Re)0.5 * c.x, x[0].y - (Re)0.5 * c.y);
+    const CT u = (SIGN > 0) ? cmk<CT>(s3 * c.y, -s3 * c.x) : cmk<CT>(-s3 * c.y, s3 * c.x);
+    x[0] = cadd(x[0], c);
+    x[1] = cadd(a, u);
+    x[2] = csub(a, u);
   } else if constexpr (R == 2 || R == 3 || R == 4) {
     bfly<R, SIGN>(x);
   } else {
@@ -507,7 +523,7 @@ __device__ __forceinline__ void rdft(CT (&x)[R]) {
 #pragma unroll
       for (int j = 0; j < m; j++) sub[r][j] = x[r + p * j];
 #pragma unroll
-    for (int r = 0; r < p; r++) rdft<m, SIGN>(sub[r]);
+    for (int r = 0; r < p; r++) rdft<m, SIGN, GAP>(sub[r]);
 #pragma unroll
     for (int k = 0; k < m; k++) {
       CT t[p];
@@ -594,8 +610,16 @@ __device__ __forceinline__ void line_tasks(int nb, Fn &&fn) {
 
 // Transform of nb lines of length N = R1 R2 R3 in shared memory, in passes of
 // radix R1, R2, R3 (R3 = 1: two passes; R2 = 1: one), a task of a pass being
-// one register DFT.  Small radices: the two-pass form with radices up to 48
-// needs 130 to 255 registers a thread and leaves 8 to 18 warps on an SM.
+// one register DFT.  FP64: small radices, as the two-pass form with radices up
+// to 48 needs 130 to 255 registers a thread and leaves 8 to 18 warps on an SM.
+//
+// FP32 (DIT): two passes, every register DFT by decimation in time (rdft)
+// whatever is known to be zero or dropped.  The phi equation weights the FP32
+// rounding by k^3, and what the rounded twiddles let through to a mode depends
+// on the factors that it passes.  Three passes of small radices with the radix
+// 3 of the direct transform last (dft_trunc) are further from 64 bits (phi of
+// one pass of 512 x 60 x 512 5.6e-6 after 5.0e-6, of 2-D 256 x 60 4.3e-7 after
+// 2.9e-7) and put the largest errors at other modes (1.4e-3 of phi's rms).
 //
 // The inverse ("inv") takes natural order and leaves X[k1 + R1 k2 + R1 R2 k3]
 // at position (k1 R2 + k2) R3 + k3; the direct one ("fwd") is its transpose,
@@ -616,7 +640,12 @@ struct Fft {
   static constexpr int RUN = fft_run(R1, R2, R3), PR = P / RUN;  // runs per pad slot
   static constexpr int LD = N + (P < N ? N / P : 0);
   static constexpr int FW = N + M, FS = R3 > 1 ? R2 : R1;
-  static_assert(R1 % 3 == 0, "the 3/2-rule gap must be whole sample rows of the first pass");
+  static constexpr bool DIT = sizeof(CT) == sizeof(float2);
+  static_assert(R1 % 3 == 0 || DIT, "the 3/2-rule gap must be whole sample rows of the first pass");
+  static_assert(R3 == 1 || !DIT, "FP32: two passes");
+  // whether sample n is a low one (n < N/3) or a high one (n > 2N/3)
+  __host__ __device__ static constexpr bool low(int n) { return n < N / 3; }
+  __host__ __device__ static constexpr bool high(int n) { return n > N / 3 * 2; }
   static_assert(P % RUN == 0 && (P == RUN || M % P == 0), "a pad slot follows whole runs");
   __device__ static __forceinline__ int sk(int n) { return P < N ? n + n / P : n; }
   static constexpr int SM = M + (P < N ? M / P : 0);  // sk(k M + n) = k SM + sk(n)
@@ -632,14 +661,6 @@ struct Fft {
 
   // slot of sample j of a second-pass task, from its first
   __host__ __device__ static constexpr int at2(int j) { return R3 > 1 ? j * R3 + j / PR : j; }
-  // The k1 of the second-pass tasks in the order of the lanes.  FP32, runs of
-  // eight padded in pairs: lines k1 and k1 + 2 are eight banks apart, k1 and
-  // k1 + 1 four, so that the two of a half warp are two apart.
-  __device__ static __forceinline__ int lane_k1(int k) {
-    if constexpr (RUN == 8 && PR == 2 && SM % 8 == 4) return k < R1 / 4 * 4 ? (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1) : k;
-    else return k;
-  }
-
   // first pass of the inverse: mk(b, n1) gives the reader of task n1 of line b,
   // rd(o, up) its sample n1 + o (o a multiple of M) in the low (n < N/3) or the
   // high third (up; n > 2N/3: 2N/3 itself is never asked for); the rest is zero
@@ -648,13 +669,24 @@ struct Fft {
     line_tasks<M, T>(nb, [&](int b, int n1) {
       const auto rd = mk(b, n1);
       CT x[R1];
+      if constexpr (R1 % 3 == 0) {
 #pragma unroll
-      for (int j = 0; j < R1; j++) {
-        if (j < Q) x[j] = rd(M * j, false);
-        else if (j > 2 * Q || (j == 2 * Q && n1 > 0)) x[j] = rd(M * j, true);
-        else x[j] = cz<CT>();
+        for (int j = 0; j < R1; j++) {
+          if (j < Q) x[j] = rd(M * j, false);
+          else if (j > 2 * Q || (j == 2 * Q && n1 > 0)) x[j] = rd(M * j, true);
+          else x[j] = cz<CT>();
+        }
+        if constexpr (DIT) rdft<R1, SIGN, true>(x);
+        else dft_gap<R1, SIGN>(x);
+      } else {  // the ends of the gap lie inside a row of samples
+#pragma unroll
+        for (int j = 0; j < R1; j++) {
+          if (low(M * j) && low(n1 + M * j)) x[j] = rd(M * j, false);
+          else if (high(M * j + M - 1) && high(n1 + M * j)) x[j] = rd(M * j, true);
+          else x[j] = cz<CT>();
+        }
+        rdft<R1, SIGN>(x);
       }
-      dft_gap<R1, SIGN>(x);
       CT *p = sm + (size_t)b * ld + sk(n1);
       const CT *t = tw + n1;
 #pragma unroll
@@ -667,7 +699,7 @@ struct Fft {
   __device__ static __forceinline__ void inv_p2(CT *sm, int nb, int ld, const CT *__restrict__ tw) {
     if constexpr (R2 > 1) {
       line_tasks<R1 * R3, T>(nb, [&](int b, int q) {
-        const int k1 = lane_k1(q / R3), n2 = q % R3;
+        const int k1 = q / R3, n2 = q % R3;
         CT *p = sm + (size_t)b * ld + k1 * SM + n2;
         const CT *t = tw + N + n2;
         CT x[R2];
@@ -721,7 +753,7 @@ struct Fft {
   __device__ static __forceinline__ void fwd_p2(CT *sm, int nb, int ld, const CT *__restrict__ tw) {
     if constexpr (R2 > 1) {
       line_tasks<R1 * R3, T>(nb, [&](int b, int q) {
-        const int k1 = lane_k1(q / R3), n2 = q % R3;
+        const int k1 = q / R3, n2 = q % R3;
         CT *p = sm + (size_t)b * ld + k1 * SM + n2;
         const CT *t = R3 > 1 ? tw + k1 * M + n2 : tw + FW + k1;
         CT x[R2];
@@ -738,11 +770,46 @@ struct Fft {
   // M j, lo for j < Q and hi for j >= 2 Q
   template <int SIGN>
   __device__ static __forceinline__ void fwd_p1(const CT *line, int n1, CT (&lo)[Q], CT (&hi)[Q]) {
+    static_assert(R1 % 3 == 0, "whole rows of outputs");
     CT x[R1];
     line += sk(n1);
 #pragma unroll
     for (int k = 0; k < R1; k++) x[k] = line[k * SM];
-    dft_trunc<R1, SIGN>(x, lo, hi);
+    if constexpr (DIT) {
+      rdft<R1, SIGN>(x);
+#pragma unroll
+      for (int j = 0; j < Q; j++) {
+        lo[j] = x[j];
+        hi[j] = x[2 * Q + j];
+      }
+    } else {
+      dft_trunc<R1, SIGN>(x, lo, hi);
+    }
+  }
+  // the same: put(o, up, v) takes the output v of index n1 + o in the low or
+  // (up) the high third
+  template <int SIGN, typename W>
+  __device__ static __forceinline__ void fwd_out(const CT *line, int n1, W &&put) {
+    if constexpr (R1 % 3 == 0) {
+      CT lo[Q], hi[Q];
+      fwd_p1<SIGN>(line, n1, lo, hi);
+#pragma unroll
+      for (int j = 0; j < Q; j++) put(M * j, false, lo[j]);
+#pragma unroll
+      for (int j = 0; j < Q; j++)
+        if (j > 0 || n1 > 0) put(M * (2 * Q + j), true, hi[j]);
+    } else {
+      CT x[R1];
+      line += sk(n1);
+#pragma unroll
+      for (int k = 0; k < R1; k++) x[k] = line[k * SM];
+      rdft<R1, SIGN>(x);
+#pragma unroll
+      for (int j = 0; j < R1; j++) {
+        if (low(M * j) && low(n1 + M * j)) put(M * j, false, x[j]);
+        else if (high(M * j + M - 1) && high(n1 + M * j)) put(M * j, true, x[j]);
+      }
+    }
   }
 };
 

@@ -1,6 +1,6 @@
 // lmc_fft_impl.cuh -- transform kernels of one lomacte RK3 substep,
-// templated on the four-step factorisation N = N1*N2 of the transform
-// length, on the complex type CT of the butterflies (and of the lines in
+// templated on the radices of the passes (FFT_RADIX, FFT_RADIX_F32), on the
+// complex type CT of the butterflies (and of the lines in
 // shared memory) and on the complex type ST of the work buffers in HBM:
 //   <double2, double2>  FP64 plain form
 //   <float2,  float2>   mixed form (FP32 transforms)
@@ -32,16 +32,14 @@ using namespace lmcd;
 namespace lmc {
 namespace LMC_FFT_NS {
 
-// The transforms of the x stage: a line is padded in whole bank rows (128 bytes
-// of samples), so that consecutive samples, which the first and the last pass
-// and the pointwise loop take, never share a bank, and the strided tasks of the
-// other passes do not either (FP32: but a third of the second pass's at 384
-// points, and that pass's at 288, 576 and 1152).  One slot per run left FP32
-// pairs of runs and FP64 runs of twelve in conflict.  With the twiddles of the
-// direct transforms in the order of the tasks (Fft) the x stage, which the L1
-// bounds, takes per step 9.14 ms after 10.23 (256 x 257 x 256, FP64, mu,
-// scalar), 12.56 after 13.97 (768 x 33), 1.70 after 2.00 (192 x 193 x 128);
-// FP32 17.6 after 18.3 (768 x 65).
+// The transforms of the x stage.  FP64: a line is padded in whole bank rows (128
+// bytes of samples), so that consecutive samples, which the first and the last
+// pass and the pointwise loop take, never share a bank, and the strided tasks of
+// the other passes do not either; one slot per run left runs of twelve in
+// conflict.  With the twiddles of the direct transforms in the order of the tasks
+// (Fft) the x stage, which the L1 bounds, takes per step 9.14 ms after 10.23
+// (256 x 257 x 256, mu, scalar), 12.56 after 13.97 (768 x 33), 1.70 after 2.00
+// (192 x 193 x 128).  FP32, whose runs are even: one slot per run.
 constexpr int x_pad(int r1, int r2, int r3, int un) {
   const int run = fft_run(r1, r2, r3);
   int p = run;
@@ -57,7 +55,7 @@ using XFft = Fft<R1, R2, R3, CT, T, x_pad(R1, R2, R3, 128 / (int)sizeof(CT))>;
 template <int R1, int R2, int R3>
 struct Geo {
   static constexpr int N = R1 * R2 * R3;
-  static constexpr int LD = Fft<R1, R2, R3>::LD;
+  static constexpr int RUN = fft_run(R1, R2, R3), LD = N + (RUN < N ? N / RUN : 0);
   static constexpr int ZB = N >= 144 ? 1 : N >= 36 ? 2 : 4;  // z lines per tile
 };
 template <int R1, int R2, int R3, bool F32>
@@ -68,10 +66,11 @@ struct XGeo {
 // Geometry of the z transforms: kx lines per block, threads of k_zinv (ZI) and
 // k_zfwd (ZF), and the stride of a line, which makes the passes with the
 // lines fastest across the lanes free of bank conflicts.  The z-physical rows
-// are touched in runs of KB values: 64 bytes from 576 points up (FP64, 1152
-// points, 768 x 33: k_zfwd 3.6 ms per step against 6.4 with 32 bytes; FP32
-// 3.9 against 4.3), 128 at 384 and 288 (256 x 257: FP64 2.9 against 3.7, FP32
-// 1.5 against 1.8), where the lines are short enough to fit; KiB at the three
+// are touched in runs of KB values: 64 bytes from 576 points up (1152 points, 768
+// x 33: k_zfwd 3.6 ms per step in FP64 against 6.4 with 32 bytes, 1.66 in FP32
+// against 1.76), 128 at 384 and 288 (FP64, 256 x 257: 2.9 against 3.7; FP32, 256 x
+// 129: k_zinv 1.87 against 2.06, k_zfwd 1.10 against 1.07), where the lines are
+// short enough to fit; KiB at the three
 // points of a 2-D grid, whose blocks are too small to be worth their launch
 // otherwise (512 x 257: k_zfwd 10 us per launch after 50, k_zinv 6 after 20).
 template <int R1, int R2, int R3, typename CT>
@@ -79,8 +78,13 @@ struct ZGeo {
   using F = Fft<R1, R2, R3, CT>;
   static constexpr int N = R1 * R2 * R3, W = sizeof(CT) == sizeof(float2) ? 2 : 1;
   static constexpr int KB = W * (N == 384 || N == 288 ? 8 : N >= 144 ? 4 : N == 3 ? 64 : 8);
-  static constexpr int ZI = W * (N == 1152 ? 192 : N == 576 ? 96 : N == 288 ? 96 : N >= 384 ? 128 : 64);
-  static constexpr int ZF = W * (N == 1152 ? (W == 2 ? 144 : 192) : N == 576 ? 144 : N == 288 ? 96 : N >= 384 ? 128 : 64);
+  // FP32: a thread for every task of the larger radix, or for half of them
+  // (256 x 129, k_zinv per step with the scalar and mu: 256 threads 1.87 ms, 384
+  // 2.13; k_zfwd 1.14 and 1.10; 192 x 129, 160 threads 1.01 and 0.42, 288 1.10
+  // and 0.45)
+  static constexpr int ZI = W == 2 ? (N == 1152 ? 288 : N == 288 ? 160 : N == 576 ? 192 : N == 768 || N == 384 ? 256 : N > 384 ? 384 : 128)
+                                   : N == 1152 ? 192 : N == 576 || N == 288 ? 96 : N >= 384 ? 128 : 64;
+  static constexpr int ZF = W == 2 ? (N == 384 ? 384 : ZI) : N == 576 ? 144 : ZI;
   static constexpr int MI = (W == 2 ? 768 : 512) / ZI, MF = (W == 2 ? 768 : 512) / ZF;
   static constexpr int UN = 128 / (int)sizeof(CT), OD = F::RUN + 1, ST = KB >= UN ? 1 : UN / KB;
   static constexpr int LD = N == 3 ? 3 : F::LD + ((ST * OD) % UN + UN - F::LD % UN) % UN;
@@ -131,9 +135,10 @@ __device__ __forceinline__ const ST *zsrc(const Dev &d, int f, int mode) {
 // spectral rows (lanes along kz), the last one writes its samples straight to
 // the z-physical rows (lanes along kx); in between the lines cross shared
 // memory once per pass.  The bound is HBM; what it takes to get near it is
-// warps in flight: 24 on an SM at 1152 points (FP32), where the two-pass form
-// with radices 36 and 32 had 12 (131 registers and 63 KB a block with its
-// staged rows).  768 x 17, four inputs: 401 MB in 131 us.
+// warps in flight: with its rows staged in shared memory the form with radices
+// 36 and 32 had 12 on an SM at 1152 points (FP32, 131 registers and 63 KB a
+// block), now it has 18.  768 x 33 with the scalar and mu, FP32: k_zinv 5.3 ms per
+// step, k_zfwd 1.7; in three passes 5.5 and 2.1.
 // mode 0: the transform inputs of the substep (in_field(i0) ..); mode 1 (2014
 // variant, FP64): T before the substep and Delta T, for d(rho)
 // (lomacte/cross.f:1760-1770); mode 2 (physical-field export, FP64): the
@@ -184,8 +189,9 @@ __global__ void __launch_bounds__(ZGeo<R1, R2, R3, CT>::ZI, ZGeo<R1, R2, R3, CT>
     rdft<RL, +1>(x);
 #pragma unroll
     for (int j = 0; j < RL; j++) {
-      // the samples stay in the transform's order, except for the export
-      const int z = q * RL + j, zr = mode == 2 ? F::nat(z) : z;
+      // the samples stay in the transform's order, except for the export and
+      // where the two z transforms may have different radices
+      const int z = q * RL + j, zr = mode == 2 || d.fft64 ? F::nat(z) : z;
       dst[(size_t)zr * d.zkn + il] = ccvt<ST>(x[j]);
     }
   }
@@ -203,7 +209,7 @@ __global__ void __launch_bounds__(ZGeo<R1, R2, R3, CT>::ZF, ZGeo<R1, R2, R3, CT>
   constexpr int ZT = ZG::ZF;
   using F = Fft<R1, R2, R3, CT, ZT>;
   using Re = typename CReal<CT>::R;
-  constexpr int KB = ZG::KB, LD = ZG::LD, N = F::N, M = F::M, Q = F::Q, SH = N / 3 + 1;
+  constexpr int KB = ZG::KB, LD = ZG::LD, N = F::N, M = F::M, SH = N / 3 + 1;
   extern __shared__ __align__(16) unsigned char smraw[];
   CT *W = (CT *)smraw;
   const CT *tw = wtwz<CT>(d);
@@ -217,7 +223,10 @@ __global__ void __launch_bounds__(ZGeo<R1, R2, R3, CT>::ZF, ZGeo<R1, R2, R3, CT>
     if (il >= nb) continue;
     ST v[RL];
 #pragma unroll
-    for (int j = 0; j < RL; j++) v[j] = __ldg(src + (size_t)(q * RL + j) * d.zkn + il);
+    for (int j = 0; j < RL; j++) {
+      const int z = q * RL + j, zr = d.fft64 ? F::nat(z) : z;  // as k_zinv wrote them
+      v[j] = __ldg(src + (size_t)zr * d.zkn + il);
+    }
     CT x[RL];
 #pragma unroll
     for (int j = 0; j < RL; j++) x[j] = ccvt<CT>(v[j]);
@@ -233,14 +242,9 @@ __global__ void __launch_bounds__(ZGeo<R1, R2, R3, CT>::ZF, ZGeo<R1, R2, R3, CT>
   const Re dn = (Re)(1.0 / (double)N);
   ST *row = wsb<ST>(d, f) + ((size_t)y * d.nkx + kx0) * d.mz;
   line_tasks<M, ZT>(nb, [&](int il, int n1) {
-    CT lo[Q], hi[Q];
-    F::template fwd_p1<-1>(W + il * LD, n1, lo, hi);
     ST *o = row + il * d.mz + n1;
-#pragma unroll
-    for (int j = 0; j < Q; j++) o[M * j] = ccvt<ST>(cscale(dn, lo[j]));
-#pragma unroll
-    for (int j = 0; j < Q; j++)
-      if (j > 0 || n1 > 0) o[M * (2 * Q + j) - SH] = ccvt<ST>(cscale(dn, hi[j]));
+    F::template fwd_out<-1>(W + il * LD, n1,
+                            [&](int k, bool up, CT v) { o[up ? k - SH : k] = ccvt<ST>(cscale(dn, v)); });
   });
 }
 
@@ -262,45 +266,71 @@ __device__ __forceinline__ CT x_pack(CT a, CT c, int n, bool up) {
 // each, nzb of them real) hold A + iB of the outputs ab(p, fa, fb) (fb < 0:
 // none).  A thread takes the tasks n and M - n together, which hold the
 // samples k and N - k of each other, and writes the retained kx of A and B.
+// Radices above 12 (FP32), whose two tasks do not fit a thread's registers,
+// pass the outputs through shared memory instead.
 template <int R1, int R2, int R3, int T, typename CT, typename ST, typename AB>
-__device__ __forceinline__ void x_out(const Dev &d, const CT *sm, int nl, size_t gt, int nzb, AB &&ab) {
+__device__ __forceinline__ void x_out(const Dev &d, CT *sm, int nl, size_t gt, int nzb, AB &&ab) {
   using F = XFft<R1, R2, R3, CT>;
   using G = Geo<R1, R2, R3>;
   using Re = typename CReal<CT>::R;
   constexpr int N = F::N, M = F::M, Q = F::Q, ZB = G::ZB;
   const Re dn = (Re)(1.0 / (double)N), hdn = (Re)(0.5 / (double)N);
-  line_tasks<(M > 1 ? M / 2 : 1), T>(nl * ZB, [&](int b, int na) {
-    const int p = b / ZB, l = b - p * ZB;
-    if (ZB > 1 && l >= nzb) return;
-    int fa, fb;
-    ab(p, fa, fb);
-    const size_t g = gt + (size_t)l * d.nkx;
-    ST *A = wzb<ST>(d, fa) + g, *B = fb >= 0 ? wzb<ST>(d, fb) + g : nullptr;
-    auto emit = [&](int k, CT c, CT q) {
-      A[k] = ccvt<ST>(cmk<CT>((c.x + q.x) * hdn, (c.y - q.y) * hdn));
-      if (B) B[k] = ccvt<ST>(cmk<CT>((c.y + q.y) * hdn, (q.x - c.x) * hdn));
-    };
-    const CT *line = sm + (size_t)b * G::LD;
-    CT la[Q], ha[Q];
-    F::template fwd_p1<-1>(line, na, la, ha);
-    if (na > 0) {
-      CT lb[Q], hb[Q];
-      F::template fwd_p1<-1>(line, M - na, lb, hb);
+  // the retained coefficient k of A and B from the samples k and N - k
+  auto emit = [&](ST *A, ST *B, int k, CT c, CT q) {
+    A[k] = ccvt<ST>(cmk<CT>((c.x + q.x) * hdn, (c.y - q.y) * hdn));
+    if (B) B[k] = ccvt<ST>(cmk<CT>((c.y + q.y) * hdn, (q.x - c.x) * hdn));
+  };
+  auto emit0 = [&](ST *A, ST *B, CT c) {
+    A[0] = ccvt<ST>(cmk<CT>(c.x * dn, 0));
+    if (B) B[0] = ccvt<ST>(cmk<CT>(c.y * dn, 0));
+  };
+  if constexpr (R1 > 12 || R1 % 3 != 0) {
+    line_tasks<M, T>(nl * ZB, [&](int b, int n1) {
+      if (ZB > 1 && b % ZB >= nzb) return;
+      CT *line = sm + (size_t)b * G::LD + F::sk(n1);  // output n1 + o at the place of sample n1 + o
+      F::template fwd_out<-1>(sm + (size_t)b * G::LD, n1, [&](int o, bool, CT v) { line[o / M * F::SM] = v; });
+    });
+    __syncthreads();
+    line_tasks<N / 3, T>(nl * ZB, [&](int b, int k) {
+      const int p = b / ZB, l = b - p * ZB;
+      if (ZB > 1 && l >= nzb) return;
+      int fa, fb;
+      ab(p, fa, fb);
+      const size_t g = gt + (size_t)l * d.nkx;
+      ST *A = wzb<ST>(d, fa) + g, *B = fb >= 0 ? wzb<ST>(d, fb) + g : nullptr;
+      const CT *line = sm + (size_t)b * G::LD;
+      if (k == 0) emit0(A, B, line[0]);
+      else emit(A, B, k, line[F::sk(k)], line[F::sk(N - k)]);
+    });
+  } else {
+    line_tasks<(M > 1 ? M / 2 : 1), T>(nl * ZB, [&](int b, int na) {
+      const int p = b / ZB, l = b - p * ZB;
+      if (ZB > 1 && l >= nzb) return;
+      int fa, fb;
+      ab(p, fa, fb);
+      const size_t g = gt + (size_t)l * d.nkx;
+      ST *A = wzb<ST>(d, fa) + g, *B = fb >= 0 ? wzb<ST>(d, fb) + g : nullptr;
+      const CT *line = sm + (size_t)b * G::LD;
+      CT la[Q], ha[Q];
+      F::template fwd_p1<-1>(line, na, la, ha);
+      if (na > 0) {
+        CT lb[Q], hb[Q];
+        F::template fwd_p1<-1>(line, M - na, lb, hb);
 #pragma unroll
-      for (int j = 0; j < Q; j++) {
-        emit(na + j * M, la[j], hb[Q - 1 - j]);
-        emit(M - na + j * M, lb[j], ha[Q - 1 - j]);
+        for (int j = 0; j < Q; j++) {
+          emit(A, B, na + j * M, la[j], hb[Q - 1 - j]);
+          emit(A, B, M - na + j * M, lb[j], ha[Q - 1 - j]);
+        }
+      } else {  // the two tasks that pair with themselves, 0 and M/2
+        emit0(A, B, la[0]);
+#pragma unroll
+        for (int j = 1; j < Q; j++) emit(A, B, j * M, la[j], ha[Q - j]);
+        F::template fwd_p1<-1>(line, M / 2, la, ha);
+#pragma unroll
+        for (int j = 0; j < Q; j++) emit(A, B, M / 2 + j * M, la[j], ha[Q - 1 - j]);
       }
-    } else {  // the two tasks that pair with themselves, 0 and M/2
-      A[0] = ccvt<ST>(cmk<CT>(la[0].x * dn, 0));
-      if (B) B[0] = ccvt<ST>(cmk<CT>(la[0].y * dn, 0));
-#pragma unroll
-      for (int j = 1; j < Q; j++) emit(j * M, la[j], ha[Q - j]);
-      F::template fwd_p1<-1>(line, M / 2, la, ha);
-#pragma unroll
-      for (int j = 0; j < Q; j++) emit(M / 2 + j * M, la[j], ha[Q - 1 - j]);
-    }
-  });
+    });
+  }
 }
 
 // The x stage: per (y, z line), inverse x transforms of the inputs, packed two
@@ -325,8 +355,8 @@ __device__ __forceinline__ void x_out(const Dev &d, const CT *sm, int nl, size_t
 // brought into the L2.  What bounds it: with nine lines a tile fills 90 KB
 // (FP32) or 180 KB (FP64) at 1152 points, so one or two blocks fit an SM and
 // the warps that hide the latencies and the barriers between the passes have
-// to come from the block: small radices (at most 12 samples in a thread's
-// registers) and a pointwise loop of one point at a time.
+// to come from the block: small radices in FP64, and a pointwise loop of one
+// point at a time.
 template <int R1, int R2, int R3, typename CT, typename ST, bool ZS, bool VS>
 __global__ void __launch_bounds__(XGeo<R1, R2, R3, sizeof(CT) == sizeof(float2)>::XT,
                                   XGeo<R1, R2, R3, sizeof(CT) == sizeof(float2)>::MINB)
@@ -899,6 +929,10 @@ struct Launch {
   }
 };
 
+// FP32 butterflies have radices of their own
+template <int N>
+using LaunchF32 = Launch<fft_radix(N, true).r1, fft_radix(N, true).r2, fft_radix(N, true).r3, float2, float2>;
+
 // register-DFT twiddles exp(-2 pi i e / R) of every block size
 inline cudaError_t upload_twiddles() {
   std::vector<double2> t;
@@ -921,7 +955,7 @@ inline cudaError_t upload_twiddles() {
 // then expands LMC_FFT_TU_BODY(suffix) to get its dispatch functions.
 #define LMC_FFT_FORMS(R1, R2, R3, CALL)                                   \
   switch (d.prec) {                                                   \
-    case 1: Launch<R1, R2, R3, float2, float2>::CALL; break;              \
+    case 1: LaunchF32<R1 * R2 * R3>::CALL; break;                         \
     case 2: Launch<R1, R2, R3, double2, float2>::CALL; break;             \
     default: Launch<R1, R2, R3, double2, double2>::CALL; break;           \
   }
@@ -930,7 +964,7 @@ inline cudaError_t upload_twiddles() {
   switch (d.prec) {                                                       \
     case 1:                                                               \
       if (d.fft64 & (BIT)) Launch<R1, R2, R3, double2, float2>::CALL;         \
-      else Launch<R1, R2, R3, float2, float2>::CALL;                          \
+      else LaunchF32<R1 * R2 * R3>::CALL;                                     \
       break;                                                              \
     case 2: Launch<R1, R2, R3, double2, float2>::CALL; break;                 \
     default: Launch<R1, R2, R3, double2, double2>::CALL; break;               \
@@ -952,7 +986,7 @@ inline cudaError_t upload_twiddles() {
 #define LMC_FFT_CASE_XS(N, R1, R2, R3) case N: return Launch<R1, R2, R3, double2, double2>::xphys_sm(zs, vs);
 #define LMC_FFT_CASE_OPT(N, R1, R2, R3)                                                         \
   if ((e = Launch<R1, R2, R3, double2, double2>::optin(limit)) != cudaSuccess) return e;        \
-  if ((e = Launch<R1, R2, R3, float2, float2>::optin(limit)) != cudaSuccess) return e;          \
+  if ((e = LaunchF32<N>::optin(limit)) != cudaSuccess) return e;                                \
   if ((e = Launch<R1, R2, R3, double2, float2>::optin(limit)) != cudaSuccess) return e;
 #define LMC_FFT_CASE_HAS(N, R1, R2, R3) case N: return true;
 

@@ -9,14 +9,26 @@ namespace lmc {
 // sweeps along y (lmc_ysweep.cuh): threads (modes) per block, and blocks of a
 // persistent grid at most
 constexpr int YS_TB = 128, YS_PERSIST = 148 * 2;
-// Radices of the transform lengths (Fft in lmc_device.cuh): the first is a
-// multiple of 3, so that the 3/2-rule gap is whole sample rows.
+// Radices of the transform lengths (Fft in lmc_device.cuh) with FP64
+// butterflies: the first is a multiple of 3, so that the 3/2-rule gap is whole
+// sample rows.
 struct FftRadix {
   int n, r1, r2, r3;
 };
 constexpr FftRadix FFT_RADIX[] = {{3, 3, 1, 1},    {24, 6, 4, 1},   {36, 6, 6, 1},   {48, 6, 8, 1},   {72, 12, 6, 1},
                                   {96, 12, 8, 1},  {144, 12, 12, 1}, {192, 12, 16, 1}, {288, 6, 6, 8},  {384, 6, 8, 8},
                                   {576, 6, 8, 12}, {768, 12, 8, 8}, {1152, 12, 8, 12}, {1536, 12, 8, 16}};
+// With FP32 butterflies: two passes, for their rounding (Fft).
+constexpr FftRadix FFT_RADIX_F32[] = {{3, 3, 1, 1},     {24, 6, 4, 1},    {36, 6, 6, 1},    {48, 8, 6, 1},    {72, 9, 8, 1},
+                                      {96, 12, 8, 1},   {144, 12, 12, 1}, {192, 16, 12, 1}, {288, 18, 16, 1}, {384, 24, 16, 1},
+                                      {576, 24, 24, 1}, {768, 32, 24, 1}, {1152, 36, 32, 1}, {1536, 48, 32, 1}};
+constexpr FftRadix fft_radix(int n, bool f32) {
+  for (const FftRadix &q : FFT_RADIX_F32)
+    if (f32 && q.n == n) return q;
+  for (const FftRadix &q : FFT_RADIX)
+    if (q.n == n) return q;
+  return FftRadix{n, n, 1, 1};
+}
 constexpr int NWB = 18;  // work-buffer slots: 12 + 6 transform inputs at most
 
 // Tables of the chunked y solves (lmc_ychunk.cuh), rows padded with zeros to
@@ -158,21 +170,21 @@ constexpr int NSTAT = 33;
 constexpr int XGRP = 32;  // z-tile groups of the physical-space sums
 // Threads of an x-stage block by transform length (f32: FP32 butterflies), and
 // the blocks per SM that its registers are sized for.  Where they were
-// measured, ms per step with the scalar and mu unless noted: 1152 FP32 256
-// threads 18.4 (320: 23.2 and 384: 20.3, the registers spill), FP64 384
-// threads 14.0 (512: 14.6, 576: 15.6); 384 FP32 128 threads 7.4 (192: 8.1,
-// 256: 9.7), FP64 192 threads 10.3 (128: 11.6, 256: 12.0); 288 FP64 without
-// them 160 threads 2.00 (192: 2.10, 256: 2.32); 144 FP32 without them six
-// blocks 0.54 (four: 0.57).
+// measured, x stage ms per step with the scalar and mu unless noted.  FP64:
+// 1152 384 threads 14.0 (512: 14.6, 576: 15.6); 384 192 threads 10.3 (128:
+// 11.6, 256: 12.0); 288 without them 160 threads 2.00 (192: 2.10, 256: 2.32).
+// FP32: 1152 (768 x 33) 256 threads 8.44 (288: 9.06); 768 (512 x 48) 160
+// threads 5.74 (192: 6.03, two blocks of 256: 5.53), without them 3.64 (3.77,
+// 4.00); 192 (128 x 129), whole steps without them, 96 threads 1.82 (128: 1.96).
 // The mixed form's partial-sum slots (Dev::mpart) hold one value per (z tile,
 // warp).
 __host__ __device__ constexpr int x_block(int n, bool f32) {
-  return n == 1536 ? 384 : n == 1152 ? (f32 ? 256 : 384) : n == 768 ? (f32 ? 192 : 384) : n == 576 ? 288
-       : n == 384 ? (f32 ? 128 : 192) : n == 288 ? (f32 ? 128 : 160) : 128;
+  return n == 1536 ? 384 : n == 1152 ? (f32 ? 256 : 384) : n == 768 ? (f32 ? 160 : 384) : n == 576 ? 288
+       : n == 384 ? (f32 ? 128 : 192) : n == 288 ? (f32 ? 128 : 160) : n == 192 && f32 ? 96 : 128;
 }
 __host__ __device__ constexpr int x_minb(int n, bool f32) {
   return n == 1536 ? 1 : n == 1152 ? (f32 ? 2 : 1) : n == 768 ? (f32 ? 3 : 1) : n == 576 ? 2
-       : n == 384 ? (f32 ? 4 : 3) : n == 288 ? 4 : f32 ? 6 : 4;
+       : n == 384 ? (f32 ? 4 : 3) : n == 288 ? 4 : n == 192 && f32 ? 8 : f32 ? 6 : 4;
 }
 
 enum {

@@ -9,10 +9,13 @@ and two on the way out and six roundings of stored values at 0.3e-7, together
 2e-7, and the solve that follows smooths.  Beside a field that is larger by the
 factor f its own line alone would add 0.9e-7 f.
 """
+import os
+
+import numpy as np
 import pytest
 
 from loma_phd_b200 import Lomacte
-from tests.helpers import case, oracle_for, rel_l2
+from tests.helpers import FIELDS, case, oracle_for, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +33,46 @@ def test_psi_at_low_density_contrast(gpu, nx, nz, s):
     o.step(2)
     e = rel_l2(psi, o.get_state()["psi"])
     assert e < 3e-7, e
+
+
+@pytest.mark.parametrize("nx,nz", [(768, 16), (16, 768)])
+def test_phi_where_the_rounding_is_largest(gpu, nx, nz):
+    """The largest errors of phi in form 1 are not random: they are what the
+    rounded twiddles let through from the energetic modes to those near the cut,
+    times k^3, and depend on the factors of the transforms (1152 points here).
+    tests/golden/mixed_rounding.npz has phi after one step at the 300 modes and
+    rows with the largest ones, from the two-pass transforms (the library of
+    commit b33f533, s = 4, Re = 400, Deltat = 0.005, ny = 33).  Other factors give
+    errors that have nothing to do with these, a relative difference of 1 and
+    more; the same factors leave only the random part: bar 1/2."""
+    gold = np.load(os.path.join(os.path.dirname(__file__), "golden", "mixed_rounding.npz"))
+    w, ref = gold[f"modes_{nx}x{nz}"], gold[f"phi_{nx}x{nz}"]
+    phi = {}
+    for prec in (0, 1):
+        p, y, st = case(nx, nz, 33, s=4.0, Re=400.0, dt=0.005, precision=prec)
+        g = Lomacte(p, y)
+        g.load_state(st)
+        g.step(1)
+        phi[prec] = g.get_state()["phi"].ravel()[w]
+        g.close()
+    off = np.linalg.norm(phi[1] - ref) / np.linalg.norm(ref - phi[0])
+    assert off < 0.5, off
+
+
+@pytest.mark.parametrize("mask", ["1", "2", "4", "5", "7"])
+def test_fft64_with_other_radices(gpu, monkeypatch, mask):
+    """Stages with FP64 butterflies beside stages with FP32 ones at lengths whose
+    radices differ between the two (72 and 288 points in x and z): nearer to the
+    FP64 oracle or as near, within the one-step bar of the mixed forms."""
+    p, y, st = case(48, 192, 17, precision=1)
+    monkeypatch.setenv("LMC_FFT64", mask)
+    g = Lomacte(p, y)
+    g.load_state(st)
+    g.step(1)
+    sg = g.get_state()
+    g.close()
+    o = oracle_for(case(48, 192, 17)[0], y, st)
+    o.step(1)
+    so = o.get_state()
+    for k in FIELDS:
+        assert rel_l2(sg[k], so[k]) < 1e-6, (k, rel_l2(sg[k], so[k]))
