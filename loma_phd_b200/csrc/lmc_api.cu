@@ -207,11 +207,13 @@ size_t sweep_scratch(int ysb, int q, const lmc::Grid &g) {
 // coefficients per row, and as many modes per block as 512 threads allow
 // (4,560 x 129, float2 buffers: 1.29 ms, 1.41 with 8 modes, 1.35 with five
 // rows; 12,192 x 193, FP64: 5.29 with 16 modes, 5.65 with 8, 5.79 with five
-// rows).
+// rows).  The scans work in whole warps, so a block has one at least: pencils of
+// up to 15 points, three five-row chunks, take nine rows and 32 modes.
 void y_geometry(lmc::Dev &d, const lmc::Grid &g) {
   d.ysb = sweep_blocks(g, d.variant);
   const bool few = !many_modes(g.nmode) && g.nmode <= FEW_MODES;
-  d.yC = few && (g.my + 4) / 5 * 8 <= 512 ? 5 : 9;
+  const int t5 = (g.my + 4) / 5 * 8;  // threads of a block of five-row chunks
+  d.yC = few && t5 >= 32 && t5 <= 512 ? 5 : 9;
   d.ync = (g.my + d.yC - 1) / d.yC;
   d.yMB = d.yC == 5 ? 8 : d.ync * 32 <= 256 ? 32 : d.ync * 16 <= 512 ? 16 : 8;
 }

@@ -282,6 +282,7 @@ __device__ __forceinline__ void scan_unit_p(int sub, int nc, const Sm<MB> &S) {
   S.G[(g * 3 + 1) * MB + ml] = e[1];
 }
 
+// A block is one whole warp at least (y_geometry):
 // the scans of slots 0 .. F1-1 (d/dy) and F1 .. F1+F2-1 (d2/dy2), or of one
 // Poisson solve, each on its own warps; between barriers
 template <int MB, int F1, int F2, bool UP>
