@@ -555,6 +555,9 @@ __device__ __forceinline__ double2 mo00(const Dev &d, int o, int j) {
   return make_double2(d.mo_cur[(size_t)o * d.my + j] / ((double)d.mgalx * (double)d.mgalz), 0.0);
 }
 
+// tables that the single operators use
+__host__ __device__ constexpr int op_tables(int op) { return op == 2 ? 2 : op == 4 ? 0 : 1; }
+
 #define LMC_YC_PROLOGUE(F, POISSON, TAB)               \
   extern __shared__ __align__(16) unsigned char raw[]; \
   const Th<C, MB> T(d, blockIdx.x);                    \
@@ -1020,42 +1023,50 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_psi(Dev d, int rk) {
   store(T, d.psi, x);
 }
 
-// single y operator on FP64 device-layout fields: 1 d/dy, 2 d2/dy2,
-// 3 Lapvdvhom (out = v, out2 = dv/dy), 4 solvepsi
-template <int C, int MB>
-__global__ void __launch_bounds__(YC_TMAX, 1) c_op(Dev d, int op, const double2 *in, double2 *out, double2 *out2) {
-  LMC_YC_PROLOGUE(2, true, 2)
-  double2 x[1][C], b[C];
+// single y operator on FP64 device-layout fields: OP 1 d/dy, 2 d2/dy2,
+// 3 Lapvdvhom (out = v, out2 = dv/dy), 4 solvepsi.  A block forms nothing but
+// its operator: with both derivatives formed for either one lmc_op_y took 0.24 ms
+// on 512 x 33 x 512 and 0.22 on 256 x 129 x 256, now 0.15 and 0.15 (d/dy; one
+// thread per mode before that 0.17 and 0.21).
+template <int C, int MB, int OP>
+__global__ void __launch_bounds__(YC_TMAX, 1) c_op(Dev d, const double2 *in, double2 *out, double2 *out2) {
+  LMC_YC_PROLOGUE(1, OP > 2, op_tables(OP))
+  double2 x[1][C];
   {
     double2 u[C + 6];
     rows_h(d, T, in, u);
-    S.tables1();
-    S.tables2();
-    if (op <= 2) {
+    if constexpr (OP == 1) {
+      S.tables1();
       d1_fwd(d, T, S, 0, u, x[0]);
-      d2_fwd(d, T, S, 1, 0.0, u, b);
+    } else if constexpr (OP == 2) {
+      S.tables2();
+      d2_fwd(d, T, S, 0, 0.0, u, x[0]);
     } else {
-      poisson(d, T, S, u, b);
+      poisson(d, T, S, u, x[0]);
     }
   }
-  if (op <= 2) {
-    d12_rest(d, T, S, x, b);
-    if (op == 1) store(T, out, x[0]);
-    else store(T, out, b);
-    return;
+  if constexpr (OP == 1) {
+    d1_rest(d, T, S, x);
+  } else if constexpr (OP == 2) {
+    scans<MB, 0, 1, false>(d, T.nc, S);
+    d2_bwd(d, T, S, 0, x[0]);
+    scans<MB, 0, 1, true>(d, T.nc, S);
+    d2_end(d, T, S, 0, x[0]);
   }
-  if (op == 4) neumann(d, T, S, b);
-  store(T, out, b);
-  if (op == 4) return;
-  put_edges(T, S, 0, b);
-  __syncthreads();
-  {
-    double2 u[C + 6];
-    with_halo(T, S, 0, b, u);
-    d1_fwd(d, T, S, 0, u, x[0]);
+  if constexpr (OP == 4) neumann(d, T, S, x[0]);
+  store(T, out, x[0]);
+  if constexpr (OP == 3) {
+    S.tables1();
+    put_edges(T, S, 0, x[0]);
+    __syncthreads();
+    {
+      double2 u[C + 6];
+      with_halo(T, S, 0, x[0], u);
+      d1_fwd(d, T, S, 0, u, x[0]);
+    }
+    d1_rest(d, T, S, x);
+    store(T, out2, x[0]);
   }
-  d1_rest(d, T, S, x);
-  store(T, out2, x[0]);
 }
 
 }  // namespace ych
@@ -1168,7 +1179,14 @@ void YC<C, MB>::psi(const Dev &d, int rk, cudaStream_t s) {
 }
 template <int C, int MB>
 void YC<C, MB>::op_y(const Dev &d, int op, const double2 *in, double2 *out, double2 *out2, cudaStream_t s) {
-  ych::go<MB>(ych::c_op<C, MB>, d, 2, true, 2, 1, 0, s, op, in, out, out2);
+  auto run = [&](auto o) {
+    constexpr int OP = decltype(o)::value;
+    ych::go<MB>(ych::c_op<C, MB, OP>, d, 1, OP > 2, ych::op_tables(OP), 1, 0, s, in, out, out2);
+  };
+  if (op == 1) run(std::integral_constant<int, 1>());
+  else if (op == 2) run(std::integral_constant<int, 2>());
+  else if (op == 3) run(std::integral_constant<int, 3>());
+  else run(std::integral_constant<int, 4>());
 }
 template <int C, int MB>
 cudaError_t YC<C, MB>::optin(int limit) {
@@ -1187,7 +1205,8 @@ cudaError_t YC<C, MB>::optin(int limit) {
                        (const void *)c_post<float2, C, MB, true, 2>, (const void *)c_post<float2, C, MB, false, 2>,
                        (const void *)c_post<double2, C, MB, true, 2>, (const void *)c_post<double2, C, MB, false, 2>,
                        (const void *)c_psi<float2, C, MB, false>, (const void *)c_psi<double2, C, MB, true>,
-                       (const void *)c_psi<double2, C, MB, false>, (const void *)c_op<C, MB>};
+                       (const void *)c_psi<double2, C, MB, false>, (const void *)c_op<C, MB, 1>,
+                       (const void *)c_op<C, MB, 2>, (const void *)c_op<C, MB, 3>, (const void *)c_op<C, MB, 4>};
   for (const void *fn : fns) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
     if (e != cudaSuccess) return e;
