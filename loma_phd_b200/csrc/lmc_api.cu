@@ -754,11 +754,14 @@ lmc::Dev block_dev(const lmc_handle *h, int r, bool xstage) {
 
 // The plane <-> line exchanges of the slab decomposition (chpl2ln /
 // chln2pl, change.f:1-143) as device copies: block r's planes of block
-// r2's lines, for the first nf z-physical fields.
-int exchange(lmc_handle *h, bool to_lines, int nf, cudaStream_t s) {
+// r2's lines, of the z-physical fields that were transformed: the inputs
+// (those that the x stage forms itself left out) or the outputs.
+int exchange(lmc_handle *h, bool to_lines, cudaStream_t s) {
   const auto &sp = h->split;
   const size_t es = h->d.prec ? sizeof(float2) : sizeof(double2), nkx = (size_t)h->d.nkx;
-  for (int f = 0; f < nf; f++)
+  const int n = to_lines ? lmc::n_zin(h->d) : lmc::n_out(h->d);
+  for (int i = 0; i < n; i++) {
+    const int f = to_lines ? lmc::in_field(h->d, i) : i;
     for (int r = 0; r < sp.n; r++)
       for (int r2 = 0; r2 < sp.n; r2++) {
         char *z = (char *)sp.Z[r][f] + (size_t)sp.l0[r2] * sp.np[r] * es;
@@ -767,6 +770,7 @@ int exchange(lmc_handle *h, bool to_lines, int nf, cudaStream_t s) {
         if (to_lines) LMC_CK(cudaMemcpy2DAsync(x, nkx * es, z, w, w, sp.nl[r2], cudaMemcpyDeviceToDevice, s));
         else LMC_CK(cudaMemcpy2DAsync(z, w, x, nkx * es, w, sp.nl[r2], cudaMemcpyDeviceToDevice, s));
       }
+  }
   return LMC_OK;
 }
 
@@ -808,7 +812,7 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
         const lmc::Dev e = block_dev(h, r, false);
         run(3, s, [&] { lmc::launch_zinv(e, s); });
       }
-      if (int rc = exchange(h, true, lmc::n_in(d), s)) return rc;
+      if (int rc = exchange(h, true, s)) return rc;
     } else {
       if (side) {
         if (!fork()) return LMC_ECUDA;
@@ -845,7 +849,7 @@ int enqueue_step(lmc_handle *h, int cfl_step, bool stats = false, bool split = f
         const lmc::Dev e = block_dev(h, r, true);
         run(4, s, [&] { lmc::launch_xphys(e, rk, do_cfl, rk == 0, s); });
       }
-      if (int rc = exchange(h, false, lmc::n_out(d), s)) return rc;
+      if (int rc = exchange(h, false, s)) return rc;
       for (int r = 0; r < h->split.n; r++) {
         const lmc::Dev e = block_dev(h, r, false);
         run(5, s, [&] { lmc::launch_zfwd(e, s); });
