@@ -152,8 +152,8 @@ int pick_chunks(int my, int &C, int &lpm, int &base, int &extra) {
   return LMC_OK;
 }
 
-// The x stage holds a tile's transform lines (and, where they fit, its
-// staged input rows) in shared memory; with the passive scalar and the
+// The x stage holds a tile's transform lines and its RHS rows in shared
+// memory; with the passive scalar and the
 // variable viscosity the lines of the largest lengths alone need more than
 // the 227 KB a B200 block can have.
 constexpr size_t SMEM_BLOCK_MAX = 227 * 1024;

@@ -1,15 +1,14 @@
 // lmc_device.cuh -- device building blocks of the lomacte substep kernels.
 //
-// y-direction operators: one warp per (kx,kz) mode.  The pencil of my
-// points is split into chunks of n in {C-1, C} consecutive points, one chunk
-// per active lane (LPM active lanes).  Banded matrix-vector products
-// exchange a halo of H points with the neighbour lanes by shuffles.  Banded
-// triangular solves run each chunk's recurrence in registers and join the
-// chunks with a Kogge-Stone scan of the affine chunk maps
-// state_out = M state_in + p.  For the mode-independent operators (the
-// compact-derivative LUs) the scan matrices are precomputed on the host, so
-// only the particular responses p travel between lanes; for the per-mode
-// Poisson LUs the 2x2 maps are built in registers.
+// y-direction operators of the 00 modes and of the no-allocation d/dy: one warp
+// per pencil.  The my points
+// are split into chunks of n in {C-1, C} consecutive points, one chunk per
+// active lane (LPM active lanes).  Banded matrix-vector products exchange a
+// halo of H points with the neighbour lanes by shuffles.  Banded triangular
+// solves run each chunk's recurrence in registers and join the chunks with a
+// Kogge-Stone scan of the affine chunk maps state_out = M state_in + p, whose
+// matrices come from the host (the compact-derivative LUs), so only the
+// particular responses p travel between lanes.
 //
 // x/z transforms: FFTs in passes of register DFTs over lines in shared memory
 // (Fft below).
@@ -101,60 +100,10 @@ __device__ __forceinline__ double tab(const double *__restrict__ T, int W, int t
   return __ldg(T + ((size_t)t * W + c) * 32 + lane);
 }
 
-// chunk <-> pencil held in shared memory (or any pointer)
-template <int C>
-__device__ __forceinline__ void cld(const double2 *p, const Lane &L, double2 (&v)[C]) {
-#pragma unroll
-  for (int t = 0; t < C; t++) v[t] = (t < L.n) ? p[L.s + t] : czero();
-}
-template <int C>
-__device__ __forceinline__ void cst(double2 *p, const Lane &L, const double2 (&v)[C]) {
-#pragma unroll
-  for (int t = 0; t < C; t++)
-    if (t < L.n) p[L.s + t] = v[t];
-}
-
-// out = band(A) * v, A rows of 2H+1 coefficients (column offsets -H..H).
-// The coefficient tables hold zeros for out-of-range columns and the halos
-// of the first/last lanes are zero.
-template <int C, int H>
-__device__ __forceinline__ void matvec(const double *__restrict__ A, const Lane &L, const double2 (&v)[C],
-                                       double2 (&out)[C]) {
-  double2 lh[H], rh[H];
-#pragma unroll
-  for (int q = 0; q < H; q++) {
-    const double2 tl = L.full ? v[C - H + q] : v[C - 1 - H + q];
-    lh[q] = shfl_up2(tl, 1);
-    rh[q] = shfl_down2(v[q], 1);
-    if (L.lane == 0) lh[q] = czero();
-    if (L.lane >= L.lpm - 1) rh[q] = czero();
-  }
-#pragma unroll
-  for (int t = 0; t < C; t++) {
-    double2 acc = czero();
-    if (t < L.n) {
-#pragma unroll
-      for (int c = 0; c < 2 * H + 1; c++) {
-        const int e = t - H + c;
-        double2 u;
-        if (e < 0) u = lh[e + H];
-        else if (e < C - 1) u = v[e];
-        else if (e == C - 1) u = L.full ? v[C - 1] : rh[0];
-        else {
-          const int i0 = (e - C < H) ? e - C : H - 1, i1 = (e - C + 1 < H) ? e - C + 1 : H - 1;
-          u = L.full ? rh[i0] : rh[i1];
-        }
-        const double w = tab(A, 2 * H + 1, t, c, L.lane);
-        acc.x = fma(w, u.x, acc.x);
-        acc.y = fma(w, u.y, acc.y);
-      }
-    }
-    out[t] = acc;
-  }
-}
-
-// In-place variant: a rolling window keeps the H original values that the
-// rows after them still need.
+// v = band(A) * v, A rows of 2H+1 coefficients (column offsets -H..H).  The
+// coefficient tables hold zeros for out-of-range columns and the halos of the
+// first/last lanes are zero; a rolling window keeps the H original values that
+// the rows after them still need.
 template <int C, int H>
 __device__ __forceinline__ void matvec_ip(const double *__restrict__ A, const Lane &L, double2 (&v)[C]) {
   double2 lh[H], rh[H];
@@ -303,107 +252,6 @@ __device__ __forceinline__ void usolve_c(double2 (&x)[C], const double *__restri
   urun<C, B>(x, Ut, L, S, true);
 }
 
-// General solves (per-mode factors): the chunk maps are built in registers.
-template <int C, int B, bool UP>
-__device__ __forceinline__ void scan_gen(double2 (&S)[B], double (&M)[B][B], int lane) {
-#pragma unroll
-  for (int s = 0; s < 5; s++) {
-    const int off = 1 << s;
-    double2 pp[B];
-    double MM[B][B];
-#pragma unroll
-    for (int d = 0; d < B; d++) pp[d] = UP ? shfl_up2(S[d], off) : shfl_down2(S[d], off);
-#pragma unroll
-    for (int r = 0; r < B; r++)
-#pragma unroll
-      for (int q = 0; q < B; q++)
-        MM[r][q] = UP ? __shfl_up_sync(LMC_FULL, M[r][q], off) : __shfl_down_sync(LMC_FULL, M[r][q], off);
-    const bool act = UP ? (lane >= off) : (lane + off < 32);
-    if (act) {
-      double nM[B][B];
-#pragma unroll
-      for (int r = 0; r < B; r++) {
-#pragma unroll
-        for (int q = 0; q < B; q++) {
-          S[r].x = fma(M[r][q], pp[q].x, S[r].x);
-          S[r].y = fma(M[r][q], pp[q].y, S[r].y);
-          double a = 0.0;
-#pragma unroll
-          for (int k = 0; k < B; k++) a = fma(M[r][k], MM[k][q], a);
-          nM[r][q] = a;
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < B; r++)
-#pragma unroll
-        for (int q = 0; q < B; q++) M[r][q] = nM[r][q];
-    }
-  }
-}
-
-template <int C, int B>
-__device__ __forceinline__ void lsolve_g(double2 (&x)[C], const double *__restrict__ Lt, const Lane &L) {
-  double2 S[B];
-#pragma unroll
-  for (int d = 0; d < B; d++) S[d] = czero();
-  lrun<C, B>(x, Lt, L, S, false);
-  double M[B][B];
-#pragma unroll
-  for (int q = 0; q < B; q++) {
-    double2 T[B];
-    double2 z[C];
-#pragma unroll
-    for (int t = 0; t < C; t++) z[t] = czero();
-#pragma unroll
-    for (int d = 0; d < B; d++) T[d] = make_double2(d == q ? 1.0 : 0.0, 0.0);
-    lrun<C, B>(z, Lt, L, T, false);
-#pragma unroll
-    for (int r = 0; r < B; r++) M[r][q] = T[r].x;
-  }
-  scan_gen<C, B, true>(S, M, L.lane);
-#pragma unroll
-  for (int d = 0; d < B; d++) {
-    S[d] = shfl_up2(S[d], 1);
-    if (L.lane == 0) S[d] = czero();
-  }
-  lrun<C, B>(x, Lt, L, S, true);
-}
-template <int C, int B>
-__device__ __forceinline__ void usolve_g(double2 (&x)[C], const double *__restrict__ Ut, const Lane &L) {
-  double2 S[B];
-#pragma unroll
-  for (int d = 0; d < B; d++) S[d] = czero();
-  urun<C, B>(x, Ut, L, S, false);
-  double M[B][B];
-#pragma unroll
-  for (int q = 0; q < B; q++) {
-    double2 T[B];
-    double2 z[C];
-#pragma unroll
-    for (int t = 0; t < C; t++) z[t] = czero();
-#pragma unroll
-    for (int d = 0; d < B; d++) T[d] = make_double2(d == q ? 1.0 : 0.0, 0.0);
-    urun<C, B>(z, Ut, L, T, false);
-#pragma unroll
-    for (int r = 0; r < B; r++) M[r][q] = T[r].x;
-  }
-  scan_gen<C, B, false>(S, M, L.lane);
-#pragma unroll
-  for (int d = 0; d < B; d++) {
-    S[d] = shfl_down2(S[d], 1);
-    if (L.lane == 31) S[d] = czero();
-  }
-  urun<C, B>(x, Ut, L, S, true);
-}
-
-__device__ __forceinline__ double2 warp_sum2(double2 v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    v.x += __shfl_xor_sync(LMC_FULL, v.x, off);
-    v.y += __shfl_xor_sync(LMC_FULL, v.y, off);
-  }
-  return v;
-}
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(LMC_FULL, v, off);

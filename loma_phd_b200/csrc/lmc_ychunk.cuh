@@ -282,9 +282,9 @@ __device__ __forceinline__ void scan_unit_p(int sub, int nc, const Sm<MB> &S) {
   S.G[(g * 3 + 1) * MB + ml] = e[1];
 }
 
-// A block is one whole warp at least (y_geometry):
 // the scans of slots 0 .. F1-1 (d/dy) and F1 .. F1+F2-1 (d2/dy2), or of one
-// Poisson solve, each on its own warps; between barriers
+// Poisson solve, each on its own warps (a block has one at least, y_geometry);
+// between barriers
 template <int MB, int F1, int F2, bool UP>
 __device__ __forceinline__ void scans(const Dev &d, int nc, const Sm<MB> &S) {
   constexpr int SUB = MB / 8;
@@ -744,8 +744,8 @@ __global__ void __launch_bounds__(YC_TMAX, 1) c_tder(Dev d) {
 // Variable viscosity: the spectral inputs of the strain rates.  In
 // physical space d(u_i)/dx_j = T d(rho u_i)/dx_j + rho u_i dT/dx_j, and the
 // stress needs d(rho u_i)/dx_j only in the symmetric sums; this kernel
-// writes d(rho v)/dy and the three off-diagonal sums (d(rho u)/dx and
-// d(rho w)/dz are formed by the inverse z transforms from rho u and rho w).
+// writes d(rho v)/dy and the three off-diagonal sums (d(rho u)/dx is formed
+// by the x stage, d(rho w)/dz by the inverse z transforms from rho w).
 // The y derivatives are deryr2's (cfdiff.f:518-601), as every first y
 // derivative of the substep.  Runs after c_assemble on the same stream.
 // The mixed forms launch one block more: its modes 0, 1, 2 are the exact

@@ -73,29 +73,6 @@ struct RdS {
   }
 };
 
-// the per-mode LU rows of one mode, streamed: L (2 multipliers) forward,
-// U (reciprocal pivot + 2) backward
-template <int K>
-struct LRows {
-  RdS<K> l0, l1;
-  __device__ __forceinline__ void start(const Dev &d, int m) {
-    const size_t n = (size_t)d.nmode;
-    l0.start(d.PLt + m, 2 * n, d.my, 1, 0);
-    l1.start(d.PLt + n + m, 2 * n, d.my, 1, 0);
-  }
-};
-template <int K>
-struct URows {
-  RdS<K> u0, u1, u2;
-  __device__ __forceinline__ void start(const Dev &d, int m) {
-    const size_t n = (size_t)d.nmode;
-    u0.start(d.PUt + m, 3 * n, d.my, -1, d.my - 1);
-    u1.start(d.PUt + n + m, 3 * n, d.my, -1, d.my - 1);
-    u2.start(d.PUt + 2 * n + m, 3 * n, d.my, -1, d.my - 1);
-  }
-};
-
-
 // a row pushed at the low end (descending sweeps)
 __device__ __forceinline__ void push_low(Win &w, double2 v) {
 #pragma unroll
@@ -405,8 +382,8 @@ __global__ void __launch_bounds__(YS_TB) t_tder(Dev d) {
 // Variable viscosity: the spectral inputs of the strain rates.  In
 // physical space d(u_i)/dx_j = T d(rho u_i)/dx_j + rho u_i dT/dx_j, and the
 // stress needs d(rho u_i)/dx_j only in the symmetric sums; this kernel
-// writes d(rho v)/dy and the three off-diagonal sums (d(rho u)/dx and
-// d(rho w)/dz are formed by the inverse z transforms from rho u and rho w).
+// writes d(rho v)/dy and the three off-diagonal sums (d(rho u)/dx is formed
+// by the x stage, d(rho w)/dz by the inverse z transforms from rho w).
 // The y derivatives are deryr2's (cfdiff.f:518-601), as every first y
 // derivative of the substep.  Runs after t_assemble on the same stream;
 // scratch fields 0, 3 and 4 hold the forward halves (1 and 2 belong to
