@@ -15,7 +15,7 @@ import numpy as np
 import pytest
 
 from loma_phd_b200 import Lomacte
-from tests.helpers import FIELDS, case, oracle_for, rel_l2
+from tests.helpers import FIELDS, case, mixing_scalar, oracle_for, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -76,3 +76,40 @@ def test_fft64_with_other_radices(gpu, monkeypatch, mask):
     so = o.get_state()
     for k in FIELDS:
         assert rel_l2(sg[k], so[k]) < 1e-6, (k, rel_l2(sg[k], so[k]))
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2])
+@pytest.mark.parametrize("nx,nz,full", [(256, 16, 1), (384, 16, 1), (512, 16, 1), (768, 16, 1), (1024, 16, 0), (16, 256, 1),
+                                        (16, 384, 1), (16, 512, 1), (16, 768, 1), (16, 1024, 1)])
+def test_long_lines(gpu, nx, nz, full, prec):
+    """Every transform length from 384 to 1536 points through one step, with the
+    scalar and mu = T^0.7 where the x stage has room for them.  Bars: FP64 1e-10;
+    the mixed forms those of the shorter lengths (up to 192 and 384 modes), 3e-6
+    and 1e-6, times the growth of what weights the rounding: k^2 in Omega_y, k^3 in
+    phi (one and a half times 1.1e-4 and 2.9e-5 at 1024 modes)."""
+    kw = dict(nx=nx, nz=nz, ny=17, **(dict(scalar=1, visc=1, sigma=0.7) if full else {}))
+    p, y, st = case(precision=prec, **kw)
+    z = mixing_scalar(p, y)
+    g = Lomacte(p, y)
+    g.load_state(st)
+    if full:
+        g.load_scalar(z)
+    g.step(1)
+    got = g.get_state()
+    if full:
+        got["Z"] = g.get_scalar()
+    g.close()
+    o = oracle_for(case(**kw)[0], y, st)
+    if full:
+        o.set_scalar(z, float(np.float32(0.7)))
+        o.set_viscosity(0.7)
+    o.step(1)
+    ref = o.get_state()
+    if full:
+        ref["Z"] = o.get_scalar()
+    bar = (1e-10, 3e-6, 1e-6)[prec]
+    n = max(nx, nz)
+    grown = {"vor": bar * (n / (n, 192, 384)[prec]) ** 2, "phi": 1.5 * (0.0, 1.1e-4, 2.9e-5)[prec] * (n / 1024) ** 3}
+    for k in FIELDS + (("Z",) if full else ()):
+        e = rel_l2(got[k], ref[k])
+        assert e < max(bar, grown.get(k, 0.0)), (k, e)
