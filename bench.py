@@ -68,7 +68,7 @@ PR = float(np.float32(0.7))  # Pr = Sc = 0.7f (main.f:569)
 # buffers take w bytes per complex value (16 in the FP64 form, 8 in the mixed
 # form).  Compulsory reads + writes of each kernel group (one profile id):
 #   zinv : 6 spectral inputs read (rho u, rho v, rho w, lap T, dT/dy, T), 8 Z written (dT/dx
-#          and, with vs, d(rho u)/dx among them, which the x stage forms now)
+#          and, with vs, d(rho u)/dx among them, which algo_bytes takes off again)
 #   xphys: 8 Z read, 11 Z written, RHS(T) physical accumulator (FP64) read + written
 #   zfwd : 11 Z read, 11 S written
 #   lapv : phi read, m_y and dm_y/dy written (+ 7 doubles/point mode tables read)
@@ -97,6 +97,14 @@ ALGO = {
     "psi": lambda S, Z, P, w, sc, vs: S * 16 + S * w + S * 7 * 8 // 2,
 }
 
+
+def algo_bytes(k, S, Z, P, w, sc, vs):
+    """Bytes of kernel group k as the kernels are: the x stage forms dT/dx and,
+    with vs, d(rho u)/dx from the lines of T and rho u, so neither is written by
+    zinv or read by xphys."""
+    return ALGO[k](S, Z, P, w, sc, vs) - ((1 + vs) * Z * w if k in ("zinv", "xphys") else 0)
+
+
 # DRAM bytes (read + write) per launch measured by ncu, by (workload, FP64
 # form): full-set captures of one launch on a case of the same x/z grid
 # with fewer y points (profiles/), scaled to a full launch by ny, as every
@@ -104,11 +112,11 @@ ALGO = {
 # not captured for that kernel.
 NCU_TRAFFIC = {
     # 768^2 x 17 (mgal 1152^2), mu = T^0.7 + scalar: profiles/kernels_xphys_mu07_scalar_768x17x768.md
-    ("large", False, 1, 1): {"xphys": (2.3682e9, 17)},
+    ("large", False, 1, 1): {"xphys": (2.3681e9, 17)},
     ("large", True, 1, 1): {"xphys": (4.0450e9, 17)},
-    # 256^2 x 65 (mgal 384^2), mu = T^0.7 + scalar, before dT/dx was formed by the x stage: profiles/kernels_xphys_mu07_scalar_256x65x256.md
-    ("medium", False, 1, 1): {"xphys": (1026.2e6, 65)},
-    ("medium", True, 1, 1): {"xphys": (1791.0e6, 65)},
+    # 256^2 x 65 (mgal 384^2), mu = T^0.7 + scalar: profiles/kernels_xphys_mu07_scalar_256x65x256.md
+    ("medium", False, 1, 1): {"xphys": (975.3e6, 65)},
+    ("medium", True, 1, 1): {"xphys": (1688.3e6, 65)},
 }
 
 MIXED_NAMES = {1: "mixed (FP32 storage and FFTs, FP64 state/solves/00 modes)",
@@ -442,7 +450,7 @@ def run_arm(a, w, prec, dev, rank, world, dist, want_e2e, steps, warmup, stats_c
     tot_ms, cnt = prof[top]
     avg_s = tot_ms / max(cnt, 1) / 1e3
     sc, vs = int(a.scalar), int(a.sigma is not None)
-    algo = ALGO[top](S, Z, P, wb, sc, vs)
+    algo = algo_bytes(top, S, Z, P, wb, sc, vs)
     peak, kind = peaks()
     achieved = algo / avg_s / 1e9
     # fraction of the timed region during which each kernel group runs; the
@@ -464,7 +472,7 @@ def run_arm(a, w, prec, dev, rank, world, dist, want_e2e, steps, warmup, stats_c
                 "traffic_source": f"ncu dram__bytes_read.sum + dram__bytes_write.sum per launch at ny={tr[1]}, "
                                   f"scaled by ny" if tr else None,
                 "algo_bytes_per_launch": algo, "avg_launch_ms": avg_s * 1e3}
-    step_bytes = 3 * sum(f(S, Z, P, wb, sc, vs) for f in ALGO.values())
+    step_bytes = 3 * sum(algo_bytes(k, S, Z, P, wb, sc, vs) for k in ALGO)
     return {"p": p, "ms": ms, "value": value, "clocks": ck, "roofline": roofline,
             "kernel_share": share, "stage_share": stage_share, "e2e": e2e, "state": state, "Z": zf, "diag": diag,
             "step_bytes": step_bytes, "stats_step": stats_step, "yop_autotune": yop,
