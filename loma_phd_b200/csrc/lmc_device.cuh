@@ -501,6 +501,8 @@ struct Fft {
   __device__ static __forceinline__ int nat(int n) {
     return n / M + R1 * ((n / R3) % R2) + R1 * R2 * (n % R3);
   }
+  // and its step along a run of the last pass
+  static constexpr int NS = R3 > 1 ? R1 * R2 : R1;
   template <int SIGN>
   __device__ static __forceinline__ CT twd(const CT *__restrict__ tw, int e) {
     const CT w = __ldg(tw + e);

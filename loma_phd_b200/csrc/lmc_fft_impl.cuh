@@ -187,13 +187,13 @@ __global__ void __launch_bounds__(ZGeo<R1, R2, R3, CT>::ZI, ZGeo<R1, R2, R3, CT>
 #pragma unroll
     for (int j = 0; j < RL; j++) x[j] = p[j];
     rdft<RL, +1>(x);
+    // the samples stay in the transform's order, except for the export and
+    // where the two z transforms may have different radices
+    const bool nat = mode == 2 || d.fft64;
+    ST *o = dst + (size_t)(nat ? F::nat(q * RL) : q * RL) * d.zkn + il;
+    const int st = (nat ? F::NS : 1) * d.zkn;
 #pragma unroll
-    for (int j = 0; j < RL; j++) {
-      // the samples stay in the transform's order, except for the export and
-      // where the two z transforms may have different radices
-      const int z = q * RL + j, zr = mode == 2 || d.fft64 ? F::nat(z) : z;
-      dst[(size_t)zr * d.zkn + il] = ccvt<ST>(x[j]);
-    }
+    for (int j = 0; j < RL; j++) o[(size_t)j * st] = ccvt<ST>(x[j]);
   }
 }
 
@@ -221,12 +221,12 @@ __global__ void __launch_bounds__(ZGeo<R1, R2, R3, CT>::ZF, ZGeo<R1, R2, R3, CT>
   for (int idx = threadIdx.x; idx < KB * (N / RL); idx += ZT) {
     const int il = idx % KB, q = idx / KB;
     if (il >= nb) continue;
+    // rows as k_zinv wrote them
+    const ST *r = src + (size_t)(d.fft64 ? F::nat(q * RL) : q * RL) * d.zkn + il;
+    const int st = (d.fft64 ? F::NS : 1) * d.zkn;
     ST v[RL];
 #pragma unroll
-    for (int j = 0; j < RL; j++) {
-      const int z = q * RL + j, zr = d.fft64 ? F::nat(z) : z;  // as k_zinv wrote them
-      v[j] = __ldg(src + (size_t)zr * d.zkn + il);
-    }
+    for (int j = 0; j < RL; j++) v[j] = __ldg(r + (size_t)j * st);
     CT x[RL];
 #pragma unroll
     for (int j = 0; j < RL; j++) x[j] = ccvt<CT>(v[j]);
