@@ -1,14 +1,14 @@
 // lmc_device.cuh -- device building blocks of the lomacte substep kernels.
 //
 // y-direction operators of the 00 modes and of the no-allocation d/dy: one warp
-// per pencil.  The my points
-// are split into chunks of n in {C-1, C} consecutive points, one chunk per
-// active lane (LPM active lanes).  Banded matrix-vector products exchange a
-// halo of H points with the neighbour lanes by shuffles.  Banded triangular
-// solves run each chunk's recurrence in registers and join the chunks with a
-// Kogge-Stone scan of the affine chunk maps state_out = M state_in + p, whose
-// matrices come from the host (the compact-derivative LUs), so only the
-// particular responses p travel between lanes.
+// per pencil.  The my points are split into chunks of n in {C-1, C}
+// consecutive points, one chunk per active lane (LPM active lanes).  Banded
+// matrix-vector products exchange a halo of H points with the neighbour lanes
+// by shuffles.  Banded triangular solves run each chunk's recurrence in
+// registers and join the chunks with a Kogge-Stone scan of the affine chunk
+// maps state_out = M state_in + p, whose matrices come from the host (the
+// compact-derivative LUs), so only the particular responses p travel between
+// lanes.
 //
 // x/z transforms: FFTs in passes of register DFTs over lines in shared memory
 // (Fft below).
